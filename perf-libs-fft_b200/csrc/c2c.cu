@@ -1,10 +1,5 @@
-// Batched complex-to-complex FP32 kernels.
+// Generic complex-to-complex FP32 tile kernel.
 //
-// c2c_reg_kernel : register engine, one transform per T = n/E threads,
-//                  G transforms per CTA; the batch-member loop of the
-//                  reference (src/batched_1d_plan.hpp:85-128 and the
-//                  planner's loop strategy, src/planner/strategies/loop.hpp:
-//                  29-35) becomes the grid.
 // c2c_tile_kernel: shared-memory engine over a tile of C transforms with
 //                  arbitrary element/transform strides; load and store each
 //                  walk the contiguous dimension so both stay coalesced.
@@ -17,35 +12,6 @@
 #include "ptx.cuh"
 
 namespace plfft_b200 {
-
-template <int E, int DIR>
-__global__ void __launch_bounds__(256) c2c_reg_kernel(const RegLaunch L) {
-  extern __shared__ float2 smem[];
-  const int T = L.t;
-  const int grp = threadIdx.x / T;
-  const int t = threadIdx.x - grp * T;
-  const int64_t b = int64_t(blockIdx.x) * L.g + grp;
-  const bool live = b < L.howmany;
-  float2* sm = smem + grp * spad_len(L.desc.n);
-
-  float2 v[E];
-  if (live) {
-    const float2* src = L.in + b * L.idist;
-#pragma unroll
-    for (int q = 0; q < E; ++q) v[q] = src[int64_t(t + T * q) * L.istride];
-  } else {
-#pragma unroll
-    for (int q = 0; q < E; ++q) v[q] = make_float2(0.f, 0.f);
-  }
-  const GroupSync sync{!(T <= 32 && (32 % T) == 0)};
-  reg_fft<E, DIR>(v, L.desc, t, T, sm, L.tw, sync);
-  if (live) {
-    float2* dst = L.out + b * L.odist;
-    const float s = L.scale;
-#pragma unroll
-    for (int q = 0; q < E; ++q) dst[int64_t(t + T * q) * L.ostride] = s == 1.f ? v[q] : cscale(v[q], s);
-  }
-}
 
 __device__ __forceinline__ int64_t tile_base(const Addr& a, int64_t g) {
   const int64_t m = g / a.ncols;
@@ -128,34 +94,11 @@ __global__ void __launch_bounds__(PLFFT_B200_TILE_THREADS(MAXE), 2) c2c_tile_ker
   }
 }
 
-int reg_smem_bytes(int n, int g) { return g * spad_len(n) * int(sizeof(float2)); }
 int tile_smem_bytes(int ld, int c) { return ld * c * int(sizeof(float2)); }
 
 template <class K>
 static cudaError_t set_smem(K kernel, int bytes) {
   return ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), bytes);
-}
-
-template <int E, int DIR>
-static cudaError_t run_reg(const RegLaunch& L, cudaStream_t st) {
-  const int smem = reg_smem_bytes(L.desc.n, L.g);
-  cudaError_t e = set_smem(c2c_reg_kernel<E, DIR>, smem);
-  if (e != cudaSuccess) return e;
-  const int64_t blocks = (L.howmany + L.g - 1) / L.g;
-  c2c_reg_kernel<E, DIR><<<dim3(unsigned(blocks)), dim3(L.t * L.g), smem, st>>>(L);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_c2c_reg(int e, int dir, const RegLaunch& L, cudaStream_t st) {
-#define PLFFT_B200_E(EV)                                                  \
-  if (e == EV) return dir < 0 ? run_reg<EV, -1>(L, st) : run_reg<EV, 1>(L, st);
-  PLFFT_B200_E(2)
-  PLFFT_B200_E(4)
-  PLFFT_B200_E(8)
-  PLFFT_B200_E(16)
-  PLFFT_B200_E(32)
-#undef PLFFT_B200_E
-  return cudaErrorInvalidValue;
 }
 
 template <int MAXE, int DIR>

@@ -23,10 +23,6 @@ namespace plfft_b200 {
 // ---------------------------------------------------------------------------
 // complex helpers
 // ---------------------------------------------------------------------------
-struct cf {
-  float x, y;
-};
-
 // Complex arithmetic on float2.  sm_100 executes two FP32 lanes per
 // instruction (FADD2/FMUL2/FFMA2), so re and im share one instruction.
 // a - b is formed as fma(b, -1, a): exact negation, one rounding, the same
@@ -47,14 +43,46 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
   return __ffma2_rn(make_float2(a.y, a.y), make_float2(b.y, b.x), t);
 }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
+
+// the same helpers on double2, and the few that build or scale either type,
+// so one codelet body serves FP32 and FP64
+__device__ __forceinline__ float2 cmake(float x, float y) { return make_float2(x, y); }
+__device__ __forceinline__ double2 cmake(double x, double y) { return make_double2(x, y); }
+// s * a + b with a real s
+__device__ __forceinline__ float2 cfma(float2 a, float s, float2 b) { return __ffma2_rn(a, make_float2(s, s), b); }
+__device__ __forceinline__ double2 cfma(double2 a, double s, double2 b) {
+  return make_double2(fma(a.x, s, b.x), fma(a.y, s, b.y));
+}
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
+}
+__device__ __forceinline__ double2 cmulc(double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, a.y * b.y), fma(a.y, b.x, -a.x * b.y));
+}
+__device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
+template <class V>
+struct ScalarOf;
+template <>
+struct ScalarOf<float2> {
+  using type = float;
+};
+template <>
+struct ScalarOf<double2> {
+  using type = double;
+};
+template <class V>
+using scalar_of = typename ScalarOf<V>::type;
+
 // multiply by (s * i) where s = +1 or -1 (compile time)
-template <int S>
-__device__ __forceinline__ float2 cmul_i(float2 a) {
-  return S > 0 ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+template <int S, class V>
+__device__ __forceinline__ V cmul_i(V a) {
+  return S > 0 ? cmake(-a.y, a.x) : cmake(a.y, -a.x);
 }
 // twiddle multiply: DIR=-1 uses the table value w, DIR=+1 uses conj(w)
-template <int DIR>
-__device__ __forceinline__ float2 twmul(float2 a, float2 w) {
+template <int DIR, class V>
+__device__ __forceinline__ V twmul(V a, V w) {
   return DIR < 0 ? cmul(a, w) : cmulc(a, w);
 }
 
@@ -114,22 +142,6 @@ constexpr cs unit_root(long long k, long long n) {
 }
 }  // namespace ce
 
-// W_n^k = exp(DIR * 2 pi i k / n) as a float2, evaluated at compile time
-template <int DIR, int N, int K>
-struct Root {
-  static constexpr ce::cs v = ce::unit_root(K, N);
-  static constexpr float re = float(v.c);
-  static constexpr float im = float(DIR * v.s);
-};
-template <int N, int K>
-struct RootCos {
-  static constexpr float v = float(ce::unit_root(K, N).c);
-};
-template <int N, int K>
-struct RootSin {
-  static constexpr float v = float(ce::unit_root(K, N).s);
-};
-
 // ---------------------------------------------------------------------------
 // static loop helper
 // ---------------------------------------------------------------------------
@@ -150,32 +162,33 @@ struct SFor {
 //   A_m = x0 + sum_k (x_k + x_{R-k}) cos(2 pi mk/R)
 //   B_m =      sum_k (x_k - x_{R-k}) sin(2 pi mk/R)
 // ---------------------------------------------------------------------------
-template <int R, int DIR>
-__device__ __forceinline__ void dft_odd(float2* v) {
+template <int R, int DIR, class V>
+__device__ __forceinline__ void dft_odd(V* v) {
+  using S = scalar_of<V>;
   constexpr int H = (R - 1) / 2;
-  float2 a[H + 1], b[H + 1];
-  float2 x0 = v[0];
-  float2 sum = x0;
+  V a[H + 1], b[H + 1];
+  V x0 = v[0];
+  V sum = x0;
 #pragma unroll
   for (int k = 1; k <= H; ++k) {
     a[k] = cadd(v[k], v[R - k]);
     b[k] = csub(v[k], v[R - k]);
     sum = cadd(sum, a[k]);
   }
-  float2 out[R];
+  V out[R];
   out[0] = sum;
   SFor<1, H + 1>::run([&](auto mc) {
     constexpr int m = decltype(mc)::value;
-    float2 A = x0, B = make_float2(0.f, 0.f);
+    V A = x0, B = cmake(S(0), S(0));
     SFor<1, H + 1>::run([&](auto kc) {
       constexpr int k = decltype(kc)::value;
-      constexpr float c = RootCos<R, (m * k) % R>::v;
-      constexpr float s = RootSin<R, (m * k) % R>::v;
-      A = __ffma2_rn(a[k], make_float2(c, c), A);
-      B = __ffma2_rn(b[k], make_float2(s, s), B);
+      constexpr S c = S(ce::unit_root((m * k) % R, R).c);
+      constexpr S s = S(ce::unit_root((m * k) % R, R).s);
+      A = cfma(a[k], c, A);
+      B = cfma(b[k], s, B);
     });
     // s*i*B with s = DIR
-    float2 iB = cmul_i<DIR>(B);
+    V iB = cmul_i<DIR>(B);
     out[m] = cadd(A, iB);
     out[R - m] = csub(A, iB);
   });
@@ -183,22 +196,22 @@ __device__ __forceinline__ void dft_odd(float2* v) {
   for (int k = 0; k < R; ++k) v[k] = out[k];
 }
 
-template <int R, int DIR>
-__device__ __forceinline__ void dft(float2* v);
+template <int R, int DIR, class V>
+__device__ __forceinline__ void dft(V* v);
 
-template <int DIR>
-__device__ __forceinline__ void dft2(float2* v) {
-  float2 a = v[0], b = v[1];
+template <int DIR, class V>
+__device__ __forceinline__ void dft2(V* v) {
+  V a = v[0], b = v[1];
   v[0] = cadd(a, b);
   v[1] = csub(a, b);
 }
 
-template <int DIR>
-__device__ __forceinline__ void dft4(float2* v) {
-  float2 t0 = cadd(v[0], v[2]);
-  float2 t1 = csub(v[0], v[2]);
-  float2 t2 = cadd(v[1], v[3]);
-  float2 t3 = cmul_i<DIR>(csub(v[1], v[3]));
+template <int DIR, class V>
+__device__ __forceinline__ void dft4(V* v) {
+  V t0 = cadd(v[0], v[2]);
+  V t1 = csub(v[0], v[2]);
+  V t2 = cadd(v[1], v[3]);
+  V t3 = cmul_i<DIR>(csub(v[1], v[3]));
   v[0] = cadd(t0, t2);
   v[2] = csub(t0, t2);
   v[1] = cadd(t1, t3);
@@ -209,13 +222,14 @@ __device__ __forceinline__ void dft4(float2* v) {
 //   n = R2*n1 + n2, k = k1 + R1*k2
 //   A[n2][k1] = DFT_R1 over n1 of x[R2 n1 + n2]; A *= W_R^{n2 k1};
 //   X[k1 + R1 k2] = DFT_R2 over n2 of A[n2][k1]
-template <int R1, int R2, int DIR>
-__device__ __forceinline__ void dft_composite(float2* v) {
+template <int R1, int R2, int DIR, class V>
+__device__ __forceinline__ void dft_composite(V* v) {
+  using S = scalar_of<V>;
   constexpr int R = R1 * R2;
-  float2 a[R];
+  V a[R];
   SFor<0, R2>::run([&](auto n2c) {
     constexpr int n2 = decltype(n2c)::value;
-    float2 t[R1];
+    V t[R1];
 #pragma unroll
     for (int n1 = 0; n1 < R1; ++n1) t[n1] = v[R2 * n1 + n2];
     dft<R1, DIR>(t);
@@ -229,17 +243,17 @@ __device__ __forceinline__ void dft_composite(float2* v) {
       } else if constexpr (4 * e == 3 * R) {
         a[n2 * R1 + k1] = cmul_i<-DIR>(t[k1]);
       } else if constexpr (2 * e == R) {
-        a[n2 * R1 + k1] = make_float2(-t[k1].x, -t[k1].y);
+        a[n2 * R1 + k1] = cmake(-t[k1].x, -t[k1].y);
       } else {
-        constexpr float wr = Root<DIR, R, e>::re;
-        constexpr float wi = Root<DIR, R, e>::im;
-        a[n2 * R1 + k1] = cmul(t[k1], make_float2(wr, wi));
+        constexpr S wr = S(ce::unit_root(e, R).c);
+        constexpr S wi = S(DIR * ce::unit_root(e, R).s);
+        a[n2 * R1 + k1] = cmul(t[k1], cmake(wr, wi));
       }
     });
   });
   SFor<0, R1>::run([&](auto k1c) {
     constexpr int k1 = decltype(k1c)::value;
-    float2 t[R2];
+    V t[R2];
 #pragma unroll
     for (int n2 = 0; n2 < R2; ++n2) t[n2] = a[n2 * R1 + k1];
     dft<R2, DIR>(t);
@@ -248,8 +262,8 @@ __device__ __forceinline__ void dft_composite(float2* v) {
   });
 }
 
-template <int R, int DIR>
-__device__ __forceinline__ void dft(float2* v) {
+template <int R, int DIR, class V>
+__device__ __forceinline__ void dft(V* v) {
   if constexpr (R == 1) {
   } else if constexpr (R == 2) {
     dft2<DIR>(v);

@@ -1,11 +1,7 @@
 // FP64 data type (complex<double> / double), reference include/plfft.h:
 // 143-154 with the FP32 conventions (docs/plfft.md:100-166).
 //
-// fp64_tile_kernel: one transform per CTA in shared memory, Stockham stages
-// of radix 2..8 with FP64 twiddles from a host table (the same stage
-// recurrence as the FP32 engine: butterfly j reads x[j + i n/R], multiplies
-// by W_{Ns R}^{(j mod Ns) i}, writes y[(j / Ns) Ns R + j mod Ns + i Ns]);
-// an optional four-step twiddle W_N^{col k} and a scale on the outputs.
+// Smooth lengths run the mixed-radix tile engine in double (mix.cuh).
 // fp64_dft_kernel: direct O(n^2) sums with exactly reduced indices, for
 // lengths without a smooth factorization.
 // fp64_real_pre / fp64_real_post: R2C and C2R through a length-n complex
@@ -14,83 +10,17 @@
 
 namespace plfft_b200 {
 
-__device__ __forceinline__ double2 dmul(double2 a, double2 b) {
-  return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ double2 dmulc(double2 a, double2 b) {  // a * conj(b)
-  return make_double2(fma(a.x, b.x, a.y * b.y), fma(a.y, b.x, -a.x * b.y));
-}
-
-template <int DIR>
-__global__ void __launch_bounds__(256) fp64_tile_kernel(const F64TileLaunch L) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int n = L.desc.n;
-  double2* buf0 = reinterpret_cast<double2*>(smraw);
-  double2* buf1 = buf0 + n;
-  const int64_t g = blockIdx.x;
-  const int64_t m = g / L.ia.ncols, col = g - (g / L.ia.ncols) * L.ia.ncols;
-  const double2* x = L.in + m * L.ia.mdist + col * L.ia.cdist;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) buf0[k] = x[int64_t(k) * L.ia.kstride];
-  __syncthreads();
-  double2* src = buf0;
-  double2* dst = buf1;
-  for (int s = 0; s < L.desc.nstages; ++s) {
-    const F64Stage st = L.desc.st[s];
-    const int R = st.radix, ns = st.ns, nb = n / R;
-    const double2* om = L.omega + st.om_off;  // exp(-2 pi i q / R), q < R
-    for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-      double2 a[8];
-      const int r = j % ns;
-      for (int i = 0; i < R; ++i) {
-        double2 v = src[j + i * nb];
-        if (ns > 1 && i > 0) {
-          const double2 w = L.tw[st.tw_off + (i - 1) * ns + r];
-          v = DIR < 0 ? dmul(v, w) : dmulc(v, w);
-        }
-        a[i] = v;
-      }
-      const int base = (j / ns) * ns * R + r;
-      for (int k = 0; k < R; ++k) {
-        double2 acc = a[0];
-        int idx = 0;
-        for (int i = 1; i < R; ++i) {
-          idx += k;
-          if (idx >= R) idx -= R;
-          acc.x += DIR < 0 ? a[i].x * om[idx].x - a[i].y * om[idx].y : a[i].x * om[idx].x + a[i].y * om[idx].y;
-          acc.y += DIR < 0 ? a[i].x * om[idx].y + a[i].y * om[idx].x : a[i].y * om[idx].x - a[i].x * om[idx].y;
-        }
-        dst[base + k * ns] = acc;
-      }
-    }
-    __syncthreads();
-    double2* t = src;
-    src = dst;
-    dst = t;
-  }
-  const int64_t om_ = g / L.oa.ncols, ocol = g - om_ * L.oa.ncols;
-  double2* y = L.out + om_ * L.oa.mdist + ocol * L.oa.cdist;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    double2 v = src[k];
-    if (L.post.n != 0) {  // W_N^{col k} = lo[e mod L] * hi[e / L]
-      const int64_t e = (col * k) % L.post.n;
-      const double2 w = dmul(L.post.lo[e % L.post.l], L.post.hi[e / L.post.l]);
-      v = DIR < 0 ? dmul(v, w) : dmulc(v, w);
-    }
-    y[int64_t(k) * L.oa.kstride] = make_double2(v.x * L.scale, v.y * L.scale);
-  }
-}
-
 // direct sums: X_k = sum_j x_j W_n^{jk}, W from an n-entry table
 template <int DIR>
-__global__ void __launch_bounds__(256) fp64_dft_kernel(const F64TileLaunch L) {
+__global__ void __launch_bounds__(256) fp64_dft_kernel(const F64DftLaunch L) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int n = L.desc.n;
+  const int n = L.n;
   double2* xs = reinterpret_cast<double2*>(smraw);
   const int64_t g = blockIdx.x;
-  const double2* x = L.in + g * L.ia.mdist;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) xs[k] = x[int64_t(k) * L.ia.kstride];
+  const double2* x = L.in + g * L.idist;
+  for (int k = threadIdx.x; k < n; k += blockDim.x) xs[k] = x[int64_t(k) * L.istride];
   __syncthreads();
-  double2* y = L.out + g * L.oa.mdist;
+  double2* y = L.out + g * L.odist;
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
     double2 acc = make_double2(0.0, 0.0);
     int idx = 0;
@@ -102,22 +32,17 @@ __global__ void __launch_bounds__(256) fp64_dft_kernel(const F64TileLaunch L) {
       idx += k;
       if (idx >= n) idx -= n;
     }
-    y[int64_t(k) * L.oa.kstride] = make_double2(acc.x * L.scale, acc.y * L.scale);
+    y[int64_t(k) * L.ostride] = make_double2(acc.x * L.scale, acc.y * L.scale);
   }
 }
 
-int fp64_tile_smem(int n) { return 2 * n * int(sizeof(double2)); }
-
-cudaError_t launch_fp64_tile(int dir, bool direct, const F64TileLaunch& L, cudaStream_t st) {
-  const int smem = direct ? L.desc.n * int(sizeof(double2)) : fp64_tile_smem(L.desc.n);
-  auto kern = direct ? (dir < 0 ? fp64_dft_kernel<-1> : fp64_dft_kernel<1>)
-                     : (dir < 0 ? fp64_tile_kernel<-1> : fp64_tile_kernel<1>);
-  {
-    const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
-    if (e != cudaSuccess) return e;
-  }
-  if (L.ntr <= 0) return cudaSuccess;
-  kern<<<dim3(unsigned(L.ntr)), dim3(256), smem, st>>>(L);
+cudaError_t launch_fp64_dft(int dir, const F64DftLaunch& L, cudaStream_t st) {
+  const int smem = L.n * int(sizeof(double2));
+  auto kern = dir < 0 ? fp64_dft_kernel<-1> : fp64_dft_kernel<1>;
+  const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+  if (e != cudaSuccess) return e;
+  if (L.howmany <= 0) return cudaSuccess;
+  kern<<<dim3(unsigned(L.howmany)), dim3(256), smem, st>>>(L);
   return cudaGetLastError();
 }
 

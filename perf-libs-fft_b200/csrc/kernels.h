@@ -30,19 +30,6 @@ struct Addr {
   int64_t ncols;
 };
 
-// Register-engine C2C launch: howmany transforms of length n, T = n/E
-// threads each, G transforms per CTA.
-struct RegLaunch {
-  const float2* in;
-  float2* out;
-  int64_t howmany;
-  int64_t istride, idist, ostride, odist;
-  int t, g;
-  float scale;
-  FftDesc desc;
-  const float2* tw;
-};
-
 // Shared-memory tile launch: C transforms per CTA, ntr transforms total,
 // `nthr` threads per CTA.
 struct TileLaunch {
@@ -253,7 +240,7 @@ struct RealFusedLaunch {
                             // 2 R2C output bins 0<k<M times 2, 3 DCT-III input
                             // element 0 (DST-III: element N-1) times 2
 };
-bool real_fused_supported(int m);
+bool real_fused_supported(int64_t m);
 int real_fused_e(int m);
 cudaError_t launch_real_fused(int kind, int m, const RealFusedLaunch& L, cudaStream_t st);
 
@@ -358,29 +345,14 @@ cudaError_t launch_half_scatter(const float* dense, void* dst, int64_t m0, int64
                                 int64_t dist, int comps, cudaStream_t st);
 
 // FP64 data type (fp64.cu)
-struct F64Stage {
-  int radix, ns, tw_off, om_off;
-};
-struct F64Desc {
-  int n, nstages;
-  F64Stage st[24];
-};
-struct TwoLevel64 {
-  const double2* lo;
-  const double2* hi;
-  int64_t n;  // 0: no four-step twiddle
-  int64_t l;
-};
-struct F64TileLaunch {
+struct F64DftLaunch {  // direct sums
   const double2* in;
   double2* out;
-  int64_t ntr;     // transforms (one per CTA)
-  Addr ia, oa;     // element addressing, as the FP32 tile launch
+  int64_t howmany;
+  int n;
+  int64_t istride, idist, ostride, odist;
   double scale;
-  F64Desc desc;    // n and stages (direct kernel: n only)
-  const double2* tw;     // stage twiddles (direct kernel: W_n^m, m < n)
-  const double2* omega;  // exp(-2 pi i q / R) for each stage radix
-  TwoLevel64 post;       // W_N^{col k} on the outputs when post.n != 0
+  const double2* tw;  // W_n^m, m < n
 };
 struct F64RealLaunch {
   const void* in;
@@ -390,8 +362,7 @@ struct F64RealLaunch {
   int c2r;
   double scale;
 };
-int fp64_tile_smem(int n);
-cudaError_t launch_fp64_tile(int dir, bool direct, const F64TileLaunch& L, cudaStream_t st);
+cudaError_t launch_fp64_dft(int dir, const F64DftLaunch& L, cudaStream_t st);
 cudaError_t launch_fp64_real(bool pre, const F64RealLaunch& L, int64_t m0, int64_t cnt, cudaStream_t st);
 
 // launch-time query caches (launch_cache.cpp)
@@ -399,9 +370,7 @@ cudaError_t ensure_dynamic_smem(const void* kernel, int bytes);
 cudaError_t cached_blocks_per_sm(const void* kernel, int threads, int smem, int* blocks);
 
 // kernel entry points (c2c.cu)
-cudaError_t launch_c2c_reg(int e, int dir, const RegLaunch& L, cudaStream_t st);
 cudaError_t launch_c2c_tile(int maxe, int dir, const TileLaunch& L, cudaStream_t st);
-int reg_smem_bytes(int n, int g);
 int tile_smem_bytes(int ld, int c);
 
 // c2c_pow2.cu

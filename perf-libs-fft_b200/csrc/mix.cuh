@@ -1,0 +1,238 @@
+// Mixed-radix tile engine: one CTA transforms a tile of `c` sequences of one
+// on-chip length, stage radices from 2..16 chosen at plan time.
+//
+// The first stage reads the user's buffer straight into registers and the
+// last one writes it straight from registers; the stages between exchange
+// through shared memory, one exchange per pair of stages.
+#pragma once
+#include <cuda_fp16.h>
+
+#include "codelets.cuh"
+#include "kernels.h"
+#include "launch_pdl.cuh"
+#include "mix.h"
+#include "ptx.cuh"
+
+namespace plfft_b200 {
+
+__device__ __forceinline__ int mix_div(int x, uint32_t mul) { return mul ? int(__umulhi(uint32_t(x), mul)) : x; }
+
+// element conversions between the user's type and the engine's
+template <class V>
+__device__ __forceinline__ V mix_cvt_in(V v) { return v; }
+__device__ __forceinline__ float2 mix_cvt_in(__half2 v) { return __half22float2(v); }
+
+// binary16 (re, im) that may lie on an odd multiple of two bytes
+struct MixHalfPair {
+  __half re, im;
+};
+__device__ __forceinline__ float2 mix_cvt_in(MixHalfPair v) { return make_float2(__half2float(v.re), __half2float(v.im)); }
+template <class U, class V>
+__device__ __forceinline__ U mix_cvt_out(V v) {
+  if constexpr (std::is_same<U, __half2>::value)
+    return __float22half2_rn(v);
+  else if constexpr (std::is_same<U, MixHalfPair>::value)
+    return MixHalfPair{__float2half_rn(v.x), __float2half_rn(v.y)};
+  else
+    return v;
+}
+
+// complex sequences of type U in global memory around an engine of type V
+template <class V, class U, int DIR>
+struct MixIoC2C {
+  const U* in;
+  U* out;
+  int64_t ics, iks, ocs, oks;
+  scalar_of<V> scale;
+  MixPost<V> post;
+  uint32_t col0;
+
+  __device__ __forceinline__ MixIoC2C(const MixLaunch<V>& L, int64_t m, int64_t col) {
+    in = static_cast<const U*>(L.in) + m * L.ia.mdist + col * L.ia.cdist;
+    out = static_cast<U*>(L.out) + m * L.oa.mdist + col * L.oa.cdist;
+    ics = L.ia.cdist;
+    iks = L.ia.kstride;
+    ocs = L.oa.cdist;
+    oks = L.oa.kstride;
+    scale = scalar_of<V>(L.scale);
+    post = L.post;
+    col0 = uint32_t(col);
+  }
+  template <int R>
+  __device__ __forceinline__ void load(int c, int j, int nb, V (&x)[R]) const {
+    const U* p = in + int64_t(c) * ics + int64_t(j) * iks;
+    const int64_t step = int64_t(nb) * iks;
+    U u[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      u[i] = *p;
+      p += step;
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) x[i] = mix_cvt_in(u[i]);
+  }
+  __device__ __forceinline__ V finish(V y, int c, int k) const {
+    if (post.lo) {
+      const uint32_t e = (col0 + uint32_t(c)) * uint32_t(k);
+      const V w = cmul(__ldg(post.lo + (e & ((1u << post.shift) - 1u))), __ldg(post.hi + (e >> post.shift)));
+      y = twmul<DIR>(y, w);
+    }
+    return cscale(y, scale);
+  }
+  template <int R>
+  __device__ __forceinline__ void store(int c, int k, int kstep, V (&x)[R]) const {
+    U* p = out + int64_t(c) * ocs + int64_t(k) * oks;
+    const int64_t step = int64_t(kstep) * oks;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      *p = mix_cvt_out<U>(finish(x[i], c, k + i * kstep));
+      p += step;
+    }
+  }
+  __device__ __forceinline__ void store1(int c, int k, V y) const {
+    out[int64_t(c) * ocs + int64_t(k) * oks] = mix_cvt_out<U>(finish(y, c, k));
+  }
+};
+
+enum MixRole { MIX_FIRST = 0, MIX_MID = 1, MIX_LAST = 2 };
+
+template <class V, int R, int DIR, int ROLE, class Io>
+__device__ __forceinline__ void mix_stage(const MixDesc& d, const MixStage& s, const V* __restrict__ tw, const V* src,
+                                          V* dst, const Io& io, int cnt) {
+  const bool cf = ROLE == MIX_FIRST ? d.cf_in : (ROLE == MIX_LAST ? d.cf_out : d.cf_mid);
+  // butterflies a thread holds at once: as many as 16 elements allow, so small
+  // radices keep as many loads in flight as large ones
+  constexpr int NB = mix_held(R);
+  const int total = s.total, nthr = blockDim.x;
+  const int tid = threadIdx.x;
+  for (int f0 = 0; f0 < total; f0 += NB * nthr) {
+    V x[NB][R];
+    bool on[NB];
+    int wpos[NB];  // shared-memory position (last stage: output index) of output 0
+    int wc[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int f = f0 + b * nthr + tid;
+      int c, j;
+      if (cf) {
+        j = mix_div(f, d.mul_c);
+        c = f - j * d.c;
+      } else {
+        c = mix_div(f, s.mul_nb);
+        j = f - c * s.nb;
+      }
+      on[b] = f < total && c < cnt;
+      int q = j, r = 0;
+      if constexpr (ROLE != MIX_FIRST) {
+        q = mix_div(j, s.mul_ns);
+        r = j - q * s.ns;
+      }
+      wc[b] = c;
+      wpos[b] = ROLE == MIX_LAST ? q * (s.ns * R) + r : c * d.ld + q * s.wblk + r;
+      // defined on every path: left undefined in an idle thread, the values of
+      // every radix stayed live across the radix switch (a kilobyte of spills)
+#pragma unroll
+      for (int i = 0; i < R; ++i) x[b][i] = cmake(scalar_of<V>(0), scalar_of<V>(0));
+      if (on[b]) {
+        if constexpr (ROLE == MIX_FIRST) {
+          io.template load<R>(c, j, s.nb, x[b]);
+        } else {
+          const V* p = src + c * d.ld + j + s.rpad * q;
+#pragma unroll
+          for (int i = 0; i < R; ++i) x[b][i] = p[i * s.rstep];
+          const V* w = tw + s.tw_off + r;
+#pragma unroll
+          for (int i = 1; i < R; ++i) x[b][i] = twmul<DIR>(x[b][i], __ldg(w + (i - 1) * s.ns));
+        }
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) dft<R, DIR>(x[b]);
+    if constexpr (ROLE == MIX_MID) {
+      if (d.inplace) __syncthreads();  // every read of the one buffer precedes its first write
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      if (!on[b]) continue;
+      if constexpr (ROLE == MIX_LAST) {
+        io.template store<R>(wc[b], wpos[b], s.ns, x[b]);
+      } else {
+        V* p = dst + wpos[b];
+#pragma unroll
+        for (int i = 0; i < R; ++i) p[i * (ROLE == MIX_FIRST ? 1 : s.ns)] = x[b][i];
+      }
+    }
+  }
+}
+
+#define PLFFT_B200_MIX_RADICES(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
+
+template <class V, int DIR, int ROLE, class Io>
+__device__ __forceinline__ void mix_dispatch(const MixDesc& d, int si, const V* tw, const V* src, V* dst,
+                                             const Io& io, int cnt) {
+  const MixStage& s = d.st[si];
+  switch (s.radix) {
+#define PLFFT_B200_CASE(R) \
+  case R:                  \
+    mix_stage<V, R, DIR, ROLE>(d, s, tw, src, dst, io, cnt); \
+    break;
+    PLFFT_B200_MIX_RADICES(PLFFT_B200_CASE)
+#undef PLFFT_B200_CASE
+    default: break;
+  }
+}
+
+template <class V>
+struct MixBounds {
+  static constexpr int threads = sizeof(V) == 8 ? 1024 : 512;
+};
+
+template <class V, int DIR, class Io>
+__global__ void __launch_bounds__(MixBounds<V>::threads, 1) mix_kernel(const __grid_constant__ MixLaunch<V> L) {
+  extern __shared__ __align__(16) unsigned char mix_smem[];
+  griddep_wait();  // launched programmatically (launch_pdl.cuh)
+  griddep_launch_dependents();
+  const MixDesc& d = L.d;
+  V* buf0 = reinterpret_cast<V*>(mix_smem);
+  V* buf1 = d.inplace ? buf0 : buf0 + d.c * d.ld;
+  const uint32_t m = blockIdx.x / L.tpm, b = blockIdx.x - m * L.tpm;
+  const int64_t col = int64_t(b) * d.c;
+  const int64_t left = L.ncols - col;
+  const int cnt = left < d.c ? int(left) : d.c;
+  const Io io(L, m, col);
+  mix_dispatch<V, DIR, MIX_FIRST>(d, 0, L.tw, buf0, buf0, io, cnt);
+  __syncthreads();
+  const int ns = d.nstages;
+  if (ns == 1) {
+    const int total = d.c * d.n;
+    for (int f = threadIdx.x; f < total; f += blockDim.x) {
+      const int k = f / d.c, c = f - k * d.c;
+      if (c < cnt) io.store1(c, k, buf0[c * d.ld + k]);
+    }
+    return;
+  }
+  V* src = buf0;
+  V* dst = buf1;
+  for (int si = 1; si < ns - 1; ++si) {
+    mix_dispatch<V, DIR, MIX_MID>(d, si, L.tw, src, dst, io, cnt);
+    __syncthreads();
+    V* t = src;
+    src = dst;
+    dst = t;
+  }
+  mix_dispatch<V, DIR, MIX_LAST>(d, ns - 1, L.tw, src, dst, io, cnt);
+}
+
+template <class V, int DIR, class Io>
+cudaError_t run_mix(const MixLaunch<V>& L, cudaStream_t st) {
+  auto* k = mix_kernel<V, DIR, Io>;
+  if (L.members <= 0 || L.ncols <= 0) return cudaSuccess;
+  const int smem = mix_smem_bytes(L.d, int(sizeof(V)));
+  const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(k), smem);
+  if (e != cudaSuccess) return e;
+  const int64_t grid = L.members * int64_t(L.tpm);
+  if (grid > 0x7fffffff) return cudaErrorInvalidValue;
+  return launch_pdl(k, dim3(unsigned(grid)), dim3(L.d.nthr), size_t(smem), st, L);
+}
+
+}  // namespace plfft_b200

@@ -1,5 +1,6 @@
 // Planner: radix factorization, device twiddle tables and C2C schedules.
 #include "plan.hpp"
+#include "plan_mix.hpp"
 
 #include <algorithm>
 #include <atomic>
@@ -117,59 +118,10 @@ static int ilog2(int64_t n) {
 }
 static bool is_pow2(int64_t n) { return n > 0 && (n & (n - 1)) == 0; }
 
-// ---------------------------------------------------------------------------
-// register-engine C2C node
-// ---------------------------------------------------------------------------
-struct RegChoice {
-  int e = 0, t = 0, g = 0;
-  std::vector<int> radices;
-};
-
 static int env_int(const char* name, int dflt) {
   const char* v = std::getenv(name);
   return v ? std::atoi(v) : dflt;
 }
-
-static bool choose_reg(int64_t n, RegChoice& rc) {
-  if (!is_pow2(n) || n < 64 || n > kMaxOnChip) return false;
-  rc.e = env_int("PLFFT_B200_REG_E", n >= 1024 ? 32 : 16);
-  if (n / rc.e > 256) return false;  // CTA limit of the register kernel
-  int64_t rest = n;
-  std::vector<int> big;
-  while (rest % rc.e == 0 && rest >= rc.e) {
-    big.push_back(rc.e);
-    rest /= rc.e;
-  }
-  rc.radices.clear();
-  if (rest > 1) rc.radices.push_back(int(rest));
-  rc.radices.insert(rc.radices.end(), big.begin(), big.end());
-  rc.t = int(n / rc.e);
-  rc.g = env_int("PLFFT_B200_REG_G", std::max(1, 256 / rc.t));
-  if (rc.g * rc.t > 256) rc.g = std::max(1, 256 / rc.t);
-  while (rc.g > 1 && reg_smem_bytes(int(n), rc.g) > 100 * 1024) rc.g /= 2;
-  return true;
-}
-
-struct C2CRegNode : Node {
-  RegLaunch base{};
-  int e = 0, dir = -1;
-  DevBuf tw;
-  std::vector<int> radices;
-  cudaError_t run(const void* in, void* out, void*, cudaStream_t st) const override {
-    RegLaunch L = base;
-    L.in = static_cast<const float2*>(in);
-    L.out = static_cast<float2*>(out);
-    return launch_c2c_reg(e, dir, L, st);
-  }
-  std::string describe() const override {
-    std::ostringstream o;
-    o << "(c2c-reg n=" << base.desc.n << " e=" << e << " t=" << base.t << " g=" << base.g
-      << " radices=";
-    for (size_t i = 0; i < radices.size(); ++i) o << (i ? "x" : "") << radices[i];
-    o << ")";
-    return o.str();
-  }
-};
 
 // ---------------------------------------------------------------------------
 // static power-of-two C2C node (bulk-copy staged, compile-time radices)
@@ -379,7 +331,10 @@ struct C2CFourStepNode : Node {
   int64_t n = 0, n1 = 0, n2 = 0;
   Layout lay{};
   int64_t chunk = 1;
-  std::unique_ptr<C2CTileNode> p1, p2;
+  std::unique_ptr<C2CTileNode> p1, p2;  // unless both factors suit the mixed-radix engine
+  MixLaunch<float2> m1{}, m2{};
+  DevBuf tw1, tw2;
+  int dir = -1;
   DevBuf lo, hi;
   size_t workspace() const override { return size_t(chunk) * size_t(n) * sizeof(float2); }
   int launches() const override { return int(2 * ((lay.howmany + chunk - 1) / chunk)); }
@@ -389,6 +344,21 @@ struct C2CFourStepNode : Node {
     float2* s = static_cast<float2*>(ws);
     for (int64_t m0 = 0; m0 < lay.howmany; m0 += chunk) {
       const int64_t cnt = std::min(chunk, lay.howmany - m0);
+      if (!p1) {
+        MixLaunch<float2> a = m1;
+        a.in = x + m0 * lay.idist;
+        a.out = s;
+        a.members = cnt;
+        cudaError_t e = launch_mix_f32(dir, a, st);
+        if (e != cudaSuccess) return e;
+        MixLaunch<float2> b = m2;
+        b.in = s;
+        b.out = y + m0 * lay.odist;
+        b.members = cnt;
+        e = launch_mix_f32(dir, b, st);
+        if (e != cudaSuccess) return e;
+        continue;
+      }
       TileLaunch a = p1->base;
       a.in = x + m0 * lay.idist;
       a.out = s;
@@ -407,7 +377,7 @@ struct C2CFourStepNode : Node {
   std::string describe() const override {
     std::ostringstream o;
     o << "(c2c-four-step n=" << n << " " << n1 << "x" << n2 << " chunk=" << chunk << " "
-      << p1->describe() << " " << p2->describe() << ")";
+      << (p1 ? p1->describe() : mix_describe(m1.d)) << " " << (p2 ? p2->describe() : mix_describe(m2.d)) << ")";
     return o.str();
   }
 };
@@ -663,12 +633,18 @@ static std::unique_ptr<Node> make_four_step(int64_t n, const Layout& lay, int di
   // pass 1: transforms g = (member, column n2), element k = n1 index
   Addr ia1{lay.idist, lay.istride, n2 * lay.istride, n2};
   Addr oa1{n, 1, n2, n2};
-  node->p1 = make_tile(n1, 0, ia1, oa1, dir, 1.0f, true, why);
   // pass 2: transforms g = (member, row k1), element k = n2 index
   Addr ia2{n, n2, 1, n1};
   Addr oa2{lay.odist, lay.ostride, n1 * lay.ostride, n1};
-  node->p2 = make_tile(n2, 0, ia2, oa2, dir, scale, false, why);
-  if (!node->p1 || !node->p2) return nullptr;
+  node->dir = dir;
+  const bool mix = mix_shape(node->m1.d, n1, n2, true, true, int(sizeof(float2)), false) &&
+                   mix_shape(node->m2.d, n2, n1, false, true, int(sizeof(float2)), false) &&
+                   n < (int64_t(1) << 32);  // the twiddle exponent col * k is 32 bits wide
+  if (!mix) {
+    node->p1 = make_tile(n1, 0, ia1, oa1, dir, 1.0f, true, why);
+    node->p2 = make_tile(n2, 0, ia2, oa2, dir, scale, false, why);
+    if (!node->p1 || !node->p2) return nullptr;
+  }
   // two-level twiddle tables for W_n^e, e < n: lo[e % L] * hi[e / L]
   int64_t L = int64_t(1) << ((ilog2(n) + 1) / 2);
   std::vector<float2> lo(L), hi((n + L - 1) / L);
@@ -678,7 +654,25 @@ static std::unique_ptr<Node> make_four_step(int64_t n, const Layout& lay, int di
     if (why) *why = "device allocation failed";
     return nullptr;
   }
-  node->p1->base.post = TwoLevel{node->lo.as<float2>(), node->hi.as<float2>(), n, int(L)};
+  if (!mix) {
+    node->p1->base.post = TwoLevel{node->lo.as<float2>(), node->hi.as<float2>(), n, int(L)};
+    return node;
+  }
+  auto pass = [&](MixLaunch<float2>& m, DevBuf& tw, const Addr& ia, const Addr& oa, double sc) {
+    m.ncols = ia.ncols;
+    m.tpm = uint32_t((ia.ncols + m.d.c - 1) / m.d.c);
+    m.ia = MixAddr{ia.mdist, ia.cdist, ia.kstride};
+    m.oa = MixAddr{oa.mdist, oa.cdist, oa.kstride};
+    m.scale = sc;
+    const bool ok = tw.upload(mix_twiddle_list<float2>(m.d)) == cudaSuccess;
+    m.tw = tw.as<float2>();
+    return ok;
+  };
+  if (!pass(node->m1, node->tw1, ia1, oa1, 1.0) || !pass(node->m2, node->tw2, ia2, oa2, scale)) {
+    if (why) *why = "device allocation failed";
+    return nullptr;
+  }
+  node->m1.post = MixPost<float2>{node->lo.as<float2>(), node->hi.as<float2>(), (ilog2(n) + 1) / 2};
   return node;
 }
 
@@ -829,29 +823,9 @@ std::unique_ptr<Node> make_c2c_node(int64_t n, const Layout& lay, int dir, float
     auto p2 = make_pow2(n, lay, dir, scale, why);
     if (p2) return p2;
   }
-  RegChoice rc;
-  if (unit && choose_reg(n, rc)) {
-    auto node = std::make_unique<C2CRegNode>();
-    std::vector<float2> tw;
-    node->base.desc = make_desc(int(n), rc.radices, tw);
-    if (node->tw.upload(tw) != cudaSuccess) {
-      if (why) *why = "device allocation failed";
-      return nullptr;
-    }
-    node->base.tw = node->tw.as<float2>();
-    node->base.howmany = lay.howmany;
-    node->base.istride = lay.istride;
-    node->base.idist = lay.idist;
-    node->base.ostride = lay.ostride;
-    node->base.odist = lay.odist;
-    node->base.t = rc.t;
-    node->base.g = rc.g;
-    node->base.scale = scale;
-    node->e = rc.e;
-    node->dir = dir;
-    node->radices = rc.radices;
-    return node;
-  }
+  // dense powers of two beyond the on-chip kernel keep the bulk-copy four-step
+  if (!(unit && is_pow2(n) && n > 8192))
+    if (auto t = make_mix_c2c<float2>(n, lay, dir, scale, false, why)) return t;
   if (n <= kMaxOnChip && is_smooth(n)) {
     Addr ia{lay.idist, 0, lay.istride, 1};
     Addr oa{lay.odist, 0, lay.ostride, 1};

@@ -1,7 +1,7 @@
 // FP64 plan nodes (kernels in fp64.cu).
 //
-// C2C: one shared-memory pass for 7-smooth n <= 4096 (radices 8, 7, 5, 4,
-// 3, 2), direct sums for other n <= 4096, a two-pass four-step for
+// C2C: the mixed-radix tile engine (mix.cuh) in double for smooth on-chip n,
+// direct sums for other n <= 4096, two mixed-radix passes for longer
 // 7-smooth n = n1 n2 with both factors <= 4096.  R2C / C2R: the real data
 // widened into a length-n complex sequence (Hermitian expansion for C2R),
 // the C2C plan, then the half spectrum (or the real parts) extracted.
@@ -10,6 +10,7 @@
 #include <sstream>
 
 #include "plan.hpp"
+#include "plan_mix.hpp"
 
 namespace plfft_b200 {
 
@@ -23,90 +24,40 @@ bool smooth7(int64_t n) {
   return n == 1;
 }
 
-std::vector<int> f64_radices(int64_t n) {
-  std::vector<int> r;
-  for (int p : {8, 7, 5, 4, 3, 2})
-    while (n % p == 0) {
-      r.push_back(p);
-      n /= p;
-    }
-  return r;
-}
-
 double2 root64(int64_t k, int64_t n) {  // exp(-2 pi i k / n)
   double c, s;
   unit_root(k, n, c, s);
   return make_double2(c, -s);
 }
 
-struct F64Tables {
-  DevBuf tw, omega;
-  F64Desc desc{};
-  bool build(int n, bool direct) {
-    desc = F64Desc{};
-    desc.n = n;
-    std::vector<double2> tw_h, om_h;
-    if (direct) {
-      for (int m = 0; m < n; ++m) tw_h.push_back(root64(m, n));
-      om_h.push_back(make_double2(1.0, 0.0));
-    } else {
-      const std::vector<int> rad = f64_radices(n);
-      if (rad.size() > 24) return false;
-      int ns = 1;
-      for (size_t s = 0; s < rad.size(); ++s) {
-        const int R = rad[s];
-        F64Stage& st = desc.st[s];
-        st.radix = R;
-        st.ns = ns;
-        st.tw_off = int(tw_h.size());
-        st.om_off = int(om_h.size());
-        if (ns > 1)
-          for (int i = 1; i < R; ++i)
-            for (int r = 0; r < ns; ++r) tw_h.push_back(root64(int64_t(r) * i, int64_t(ns) * R));
-        for (int q = 0; q < R; ++q) om_h.push_back(root64(q, R));
-        ns *= R;
-      }
-      desc.nstages = int(rad.size());
-      if (tw_h.empty()) tw_h.push_back(make_double2(1.0, 0.0));
-    }
-    return tw.upload(tw_h) == cudaSuccess && omega.upload(om_h) == cudaSuccess;
-  }
-};
-
+// n two-pass (n = n1 n2, mixed-radix tiles) or, with n2 == 0, direct sums
 struct F64C2CNode : Node {
-  int64_t n = 0, n1 = 0, n2 = 0, chunk = 1;  // n2 == 0: one pass of length n
+  int64_t n = 0, n1 = 0, n2 = 0, chunk = 1;
   int dir = -1;
-  bool direct = false;
   Layout lay{};
   double scale = 1.0;
-  F64Tables t1, t2;
-  DevBuf lo, hi;
+  MixLaunch<double2> p1{}, p2{};
+  DevBuf tw1, tw2, lo, hi;
   size_t workspace() const override { return n2 ? size_t(chunk * n) * sizeof(double2) : 0; }
   int launches() const override { return n2 ? int(2 * ((lay.howmany + chunk - 1) / chunk)) : 1; }
-  F64TileLaunch pass(const F64Tables& t, const void* in, void* out, int64_t ntr, Addr ia, Addr oa, double sc,
-                     TwoLevel64 post) const {
-    return F64TileLaunch{static_cast<const double2*>(in), static_cast<double2*>(out), ntr, ia, oa, sc, t.desc,
-                         t.tw.as<double2>(), t.omega.as<double2>(), post};
-  }
   cudaError_t run(const void* in, void* out, void* ws, cudaStream_t st) const override {
-    const TwoLevel64 none{nullptr, nullptr, 0, 1};
-    if (!n2) {
-      Addr ia{lay.idist, 0, lay.istride, 1}, oa{lay.odist, 0, lay.ostride, 1};
-      return launch_fp64_tile(dir, direct, pass(t1, in, out, lay.howmany, ia, oa, scale, none), st);
-    }
     const auto* x = static_cast<const double2*>(in);
     auto* y = static_cast<double2*>(out);
-    auto* s = static_cast<double2*>(ws);
-    const TwoLevel64 tw2{lo.as<double2>(), hi.as<double2>(), n, int64_t(std::ceil(std::sqrt(double(n))))};
+    if (!n2) {
+      const F64DftLaunch L{x,          y,           lay.howmany, int(n), lay.istride, lay.idist,
+                           lay.ostride, lay.odist, scale,       tw1.as<double2>()};
+      return launch_fp64_dft(dir, L, st);
+    }
     for (int64_t m0 = 0; m0 < lay.howmany; m0 += chunk) {
-      const int64_t cnt = std::min(chunk, lay.howmany - m0);
-      // pass 1: columns (member, n2 index) of length n1, times W_n^{col k}
-      Addr ia1{lay.idist, lay.istride, n2 * lay.istride, n2}, oa1{n, 1, n2, n2};
-      cudaError_t e = launch_fp64_tile(dir, false, pass(t1, x + m0 * lay.idist, s, cnt * n2, ia1, oa1, 1.0, tw2), st);
+      MixLaunch<double2> a = p1, b = p2;
+      a.members = b.members = std::min(chunk, lay.howmany - m0);
+      a.in = x + m0 * lay.idist;
+      a.out = ws;
+      cudaError_t e = launch_mix_f64(dir, a, st);
       if (e != cudaSuccess) return e;
-      // pass 2: rows (member, n1 index) of length n2, written transposed
-      Addr ia2{n, n2, 1, n1}, oa2{lay.odist, lay.ostride, n1 * lay.ostride, n1};
-      e = launch_fp64_tile(dir, false, pass(t2, s, y + m0 * lay.odist, cnt * n1, ia2, oa2, scale, none), st);
+      b.in = ws;
+      b.out = y + m0 * lay.odist;
+      e = launch_mix_f64(dir, b, st);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -115,9 +66,10 @@ struct F64C2CNode : Node {
     std::ostringstream o;
     o << "(c2c-fp64 n=" << n;
     if (n2)
-      o << " four-step " << n1 << "x" << n2 << " chunk=" << chunk;
+      o << " four-step " << n1 << "x" << n2 << " chunk=" << chunk << " " << mix_describe(p1.d) << " "
+        << mix_describe(p2.d);
     else
-      o << (direct ? " direct sums" : " shared-memory Stockham");
+      o << " direct sums";
     o << ")";
     return o.str();
   }
@@ -155,14 +107,18 @@ struct F64RealNode : Node {
 }  // namespace
 
 std::unique_ptr<Node> make_fp64_c2c(int64_t n, const Layout& lay, int dir, double scale, std::string* why) {
+  // 7-smooth n, and the 13-smooth ones the direct sums would take
+  if (smooth7(n) || (is_smooth(n) && n <= kF64MaxOnChip))
+    if (auto t = make_mix_c2c<double2>(n, lay, dir, scale, false, why)) return t;
   auto node = std::make_unique<F64C2CNode>();
   node->n = n;
   node->dir = dir;
   node->lay = lay;
   node->scale = scale;
   if (n <= kF64MaxOnChip) {
-    node->direct = !smooth7(n);
-    if (!node->t1.build(int(n), node->direct)) return nullptr;
+    std::vector<double2> tw(n);
+    for (int64_t m = 0; m < n; ++m) tw[m] = root64(m, n);
+    if (node->tw1.upload(tw) != cudaSuccess) return nullptr;
     return node;
   }
   if (!smooth7(n)) {
@@ -177,15 +133,33 @@ std::unique_ptr<Node> make_fp64_c2c(int64_t n, const Layout& lay, int dir, doubl
     if (why) *why = "FP64 length has no four-step split with factors <= 4096";
     return nullptr;
   }
-  node->n1 = best;
-  node->n2 = n / best;
+  const int64_t n1 = node->n1 = best, n2 = node->n2 = n / best;
   node->chunk = std::max<int64_t>(1, std::min<int64_t>(lay.howmany, (int64_t(256) << 20) / (n * 16)));
-  if (!node->t1.build(int(node->n1), false) || !node->t2.build(int(node->n2), false)) return nullptr;
-  const int64_t L = int64_t(std::ceil(std::sqrt(double(n))));
+  // pass 1: columns (member, n2 index) of length n1, times W_n^{col k};
+  // pass 2: rows (member, n1 index) of length n2, written transposed
+  if (!mix_shape(node->p1.d, n1, n2, true, true, int(sizeof(double2)), false) ||
+      !mix_shape(node->p2.d, n2, n1, false, true, int(sizeof(double2)), false) ||
+      node->tw1.upload(mix_twiddle_list<double2>(node->p1.d)) != cudaSuccess ||
+      node->tw2.upload(mix_twiddle_list<double2>(node->p2.d)) != cudaSuccess)
+    return nullptr;
+  int shift = 0;
+  while ((int64_t(1) << (2 * shift)) < n) ++shift;
+  const int64_t L = int64_t(1) << shift;
   std::vector<double2> lo(L), hi((n + L - 1) / L);
   for (int64_t i = 0; i < L; ++i) lo[i] = root64(i, n);
   for (size_t i = 0; i < hi.size(); ++i) hi[i] = root64(int64_t(i) * L, n);
   if (node->lo.upload(lo) != cudaSuccess || node->hi.upload(hi) != cudaSuccess) return nullptr;
+  auto pass = [](MixLaunch<double2>& m, int64_t ncols, MixAddr ia, MixAddr oa, double sc, const DevBuf& tw) {
+    m.ncols = ncols;
+    m.tpm = uint32_t((ncols + m.d.c - 1) / m.d.c);
+    m.ia = ia;
+    m.oa = oa;
+    m.scale = sc;
+    m.tw = tw.as<double2>();
+  };
+  pass(node->p1, n2, MixAddr{lay.idist, lay.istride, n2 * lay.istride}, MixAddr{n, 1, n2}, 1.0, node->tw1);
+  pass(node->p2, n1, MixAddr{n, n2, 1}, MixAddr{lay.odist, lay.ostride, n1 * lay.ostride}, scale, node->tw2);
+  node->p1.post = MixPost<double2>{node->lo.as<double2>(), node->hi.as<double2>(), shift};
   return node;
 }
 

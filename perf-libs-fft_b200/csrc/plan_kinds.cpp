@@ -5,6 +5,8 @@
 // follow docs/plfft.md:100-166.
 #include "plan_kinds.hpp"
 
+#include "plan_mix.hpp"
+
 #include <cstring>
 
 namespace plfft_b200 {
@@ -44,6 +46,24 @@ static int r2r_wrap_kind(int payload) {
   return map[payload];
 }
 
+// May the members of an aliased batch be transformed one CTA at a time, each
+// member's output written as soon as its own tile is read?  Yes when the
+// outputs of a member lie where its inputs do; other in-place layouts keep
+// the schedules that read the whole batch before the first write.
+static bool member_in_place(const ConfigData& c, const Layout& lay) {
+  if (c.alias != PLFFT_IO_MAY_ALIAS || lay.howmany == 1) return true;
+  int64_t nin = 0, nout = 0;
+  bool ic = false, oc = false;
+  io_counts(c, nin, nout, ic, oc);
+  return lay.istride == lay.ostride && lay.idist * (ic ? 2 : 1) == lay.odist * (oc ? 2 : 1);
+}
+
+// fused kind of an R2R payload, or -1
+static int r2r_fused_kind(int payload) {
+  static const int map[] = {-1, FR_DCT2, FR_DCT3, FR_DCT4, -1, FR_DST2, FR_DST3, FR_DST4, FR_DHT, FR_R2HC, FR_HC2R};
+  return map[payload];
+}
+
 // device schedule for configuration c over the batch layout lay; tune:
 // allow plan-time autotuning (rigor above ESTIMATE)
 static std::unique_ptr<Node> make_root(const ConfigData& c, const Layout& lay, bool tune, std::string* why,
@@ -59,38 +79,18 @@ static std::unique_ptr<Node> make_root(const ConfigData& c, const Layout& lay, b
           root = autotune_c2c(c, lay, why, note);
         break;
       case TKind::R2C:
-        if (tune && c.rigor != PLFFT_ESTIMATE) {
-          root = autotune_real(c, lay, FR_R2C, RW_R2C, why, note);
-          break;
-        }
-        root = make_real_fused_node(FR_R2C, c.n, lay, scale);
-        if (!root) root = make_realwrap_node(RW_R2C, c.n, lay, scale, why);
-        break;
       case TKind::C2R:
-        if (tune && c.rigor != PLFFT_ESTIMATE) {
-          root = autotune_real(c, lay, FR_C2R, RW_C2R, why, note);
-          break;
-        }
-        root = make_real_fused_node(FR_C2R, c.n, lay, scale);
-        if (!root) root = make_realwrap_node(RW_C2R, c.n, lay, scale, why);
-        break;
       case TKind::R2R: {
+        const int wrap = c.kind == TKind::R2C ? RW_R2C : (c.kind == TKind::C2R ? RW_C2R : r2r_wrap_kind(c.payload));
+        int fused = c.kind == TKind::R2C ? FR_R2C : (c.kind == TKind::C2R ? FR_C2R : r2r_fused_kind(c.payload));
+        // the power-of-two kernel's lengths have always run member by member
+        if (!(c.n % 2 == 0 && real_fused_supported(c.n / 2)) && !member_in_place(c, lay)) fused = -1;
         if (tune && c.rigor != PLFFT_ESTIMATE) {
-          static const int fused_of[] = {-1, FR_DCT2, FR_DCT3, FR_DCT4, -1, FR_DST2,
-                                         FR_DST3, FR_DST4, FR_DHT, FR_R2HC, FR_HC2R};
-          root = autotune_real(c, lay, fused_of[c.payload], r2r_wrap_kind(c.payload), why, note);
+          root = autotune_real(c, lay, fused, wrap, why, note);
           break;
         }
-        if (c.payload == PLFFT_R2R_DCT_2) root = make_real_fused_node(FR_DCT2, c.n, lay, scale);
-        if (c.payload == PLFFT_R2R_DST_2) root = make_real_fused_node(FR_DST2, c.n, lay, scale);
-        if (c.payload == PLFFT_R2R_DCT_3) root = make_real_fused_node(FR_DCT3, c.n, lay, scale);
-        if (c.payload == PLFFT_R2R_DST_3) root = make_real_fused_node(FR_DST3, c.n, lay, scale);
-        if (c.payload == PLFFT_R2R_DCT_4) root = make_real_fused_node(FR_DCT4, c.n, lay, scale);
-        if (c.payload == PLFFT_R2R_DST_4) root = make_real_fused_node(FR_DST4, c.n, lay, scale);
-        if (c.payload == PLFFT_R2R_R2HC) root = make_real_fused_node(FR_R2HC, c.n, lay, scale);
-        if (c.payload == PLFFT_R2R_HC2R) root = make_real_fused_node(FR_HC2R, c.n, lay, scale);
-        if (c.payload == PLFFT_R2R_DHT) root = make_real_fused_node(FR_DHT, c.n, lay, scale);
-        if (!root) root = make_realwrap_node(r2r_wrap_kind(c.payload), c.n, lay, scale, why);
+        if (fused >= 0) root = make_real_fused_node(fused, c.n, lay, scale);
+        if (!root) root = make_realwrap_node(wrap, c.n, lay, scale, why);
         break;
       }
     }
@@ -172,6 +172,10 @@ struct HalfIoNode : Node {
 };
 
 static std::unique_ptr<Node> make_half_node(const ConfigData& c, const Layout& lay, std::string* why) {
+  // C2C of an on-chip smooth length: binary16 loads and stores in the
+  // transform itself (one launch, 8 bytes per element instead of 40)
+  if (c.kind == TKind::C2C && member_in_place(c, lay))
+    if (auto t = make_mix_c2c<float2>(c.n, lay, c.payload, c.scale, true, why)) return t;
   int64_t nin = 0, nout = 0;
   bool ic = false, oc = false;
   io_counts(c, nin, nout, ic, oc);

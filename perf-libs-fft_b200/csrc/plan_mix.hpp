@@ -1,0 +1,40 @@
+// Planner interface of the mixed-radix tile engine (plan_mix.cpp).
+#pragma once
+#include <memory>
+#include <string>
+#include <vector>
+
+#include "mix.h"
+#include "plan.hpp"
+
+namespace plfft_b200 {
+
+// radices 2..16 whose product is n, cheapest stage list first found; empty
+// if n has a prime factor above 13
+std::vector<int> mix_radices(int64_t n, int max_radix);
+// radices, tile width, threads and buffers for length n and `ncols`
+// transforms; c_req > 0 asks for a tile width.  False: not on chip.
+// staged: the last stage's results go to shared memory, not to the user's
+// buffer.
+bool mix_shape(MixDesc& d, int64_t n, int64_t ncols, bool cf_in, bool cf_out, int elem_bytes, bool staged,
+               int c_req = 0);
+// stages and pads of length n (1: no stage), then a tile of exactly c such
+// transforms for a CTA of `threads` threads and a shared-memory budget of
+// max_elems complex FP32, any stage of which may run from shared memory to
+// shared memory (false: does not fit)
+bool mix_tile_layout(MixDesc& d, int n, int max_radix);
+bool mix_tile_set(MixDesc& d, int c, int threads, int max_elems);
+template <class V>
+std::vector<V> mix_twiddle_list(const MixDesc& d);
+std::string mix_describe(const MixDesc& d);
+
+// one-pass C2C of a strided batch (half: binary16 buffers, V = float2);
+// nullptr when n is not a supported on-chip length
+template <class V>
+std::unique_ptr<Node> make_mix_c2c(int64_t n, const Layout& lay, int dir, double scale, bool half, std::string* why);
+
+// one-pass real transform (FusedRealKind) of even n = 2M with on-chip smooth
+// M, unit strides; nullptr otherwise
+std::unique_ptr<Node> make_mix_real(int kind, int64_t n, const Layout& lay, float scale, int wmode);
+
+}  // namespace plfft_b200

@@ -5,6 +5,7 @@
 #include <sstream>
 
 #include "plan.hpp"
+#include "plan_mix.hpp"
 
 namespace plfft_b200 {
 
@@ -273,8 +274,10 @@ struct RealFusedNode : Node {
 
 std::unique_ptr<Node> make_real_fused_node(int kind, int64_t n, const Layout& lay, float scale, int wmode, int g_override,
                                            int e_override) {
-  if (n % 2 || !real_fused_supported(int(n / 2)) || lay.istride != 1 || lay.ostride != 1) return nullptr;
+  if (n % 2 || lay.istride != 1 || lay.ostride != 1) return nullptr;
   if (std::getenv("PLFFT_B200_NO_FUSED_REAL")) return nullptr;
+  if (!real_fused_supported(n / 2))
+    return std::getenv("PLFFT_B200_NO_REAL_HALF") ? nullptr : make_mix_real(kind, n, lay, scale, wmode);
   const int m = int(n / 2);
   int e = real_fused_e(m);
   if (const char* v = std::getenv("PLFFT_B200_RF_E"))  // launch-shape experiments
@@ -338,7 +341,9 @@ std::vector<std::unique_ptr<Node>> make_real_candidates(int fused_kind, int wrap
   std::vector<std::unique_ptr<Node>> out;
   std::string why;
   auto fused = fused_kind >= 0 ? make_real_fused_node(fused_kind, n, lay, scale) : nullptr;
-  if (fused) {
+  if (fused && !real_fused_supported(n / 2)) {
+    out.push_back(std::move(fused));
+  } else if (fused) {
     const int g0 = static_cast<RealFusedNode*>(fused.get())->base.g;
     const int e0 = static_cast<RealFusedNode*>(fused.get())->base.e;
     out.push_back(std::move(fused));

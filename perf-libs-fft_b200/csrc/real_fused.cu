@@ -16,7 +16,7 @@ int real_fused_e(int m) {
   return 32;
 }
 
-bool real_fused_supported(int m) { return m >= 64 && m <= 8192 && (m & (m - 1)) == 0; }
+bool real_fused_supported(int64_t m) { return m >= 64 && m <= 8192 && (m & (m - 1)) == 0; }
 
 cudaError_t launch_real_fused(int kind, int m, const RealFusedLaunch& L, cudaStream_t st) {
   if (!real_fused_supported(m)) return cudaErrorInvalidValue;

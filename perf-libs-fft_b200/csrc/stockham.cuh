@@ -16,13 +16,9 @@
 // (forward sign; backward conjugates at use), so lanes with consecutive j
 // read consecutive entries.
 //
-// Two engines:
-//  * RegFFT<E>: each of T = N/E threads keeps E elements in registers.  The
-//    first stage reads global memory directly and the last stage leaves the
-//    result in registers, so an N = R0*R1 transform costs one shared-memory
-//    exchange.  Requires every radix to divide E.
-//  * smem_fft<MAXE>: general engine; a CTA holds C transforms in shared
-//    memory and every stage is a read-all / barrier / write-all pass.
+// smem_fft<MAXE> holds C transforms in shared memory and every stage is a
+// read-all / barrier / write-all pass.  (One-pass lengths run the mixed-radix
+// engine of mix.cuh or the compile-time lists of pow2_stages.cuh.)
 #pragma once
 #include "codelets.cuh"
 #include "stockham_desc.h"
@@ -41,102 +37,6 @@ __device__ __forceinline__ int spad(int p) { return p + (p >> 4); }
 
 __device__ __forceinline__ int div_ns(int j, const Stage& s) {
   return s.ns_shift >= 0 ? (j >> s.ns_shift) : (j / s.ns);
-}
-
-// ===========================================================================
-// Register engine
-// ===========================================================================
-template <int E, int R, int DIR>
-__device__ __forceinline__ void reg_butterflies(float2 (&v)[E], int t, int T, const Stage& s,
-                                                const float2* __restrict__ tw) {
-  constexpr int M = E / R;
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    float2 x[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) x[i] = v[m + M * i];
-    if (s.ns > 1) {
-      const int j = t + T * m;
-      const int r = j - div_ns(j, s) * s.ns;
-      const float2* w = tw + s.tw_off + r;
-#pragma unroll
-      for (int i = 1; i < R; ++i) x[i] = twmul<DIR>(x[i], __ldg(w + (i - 1) * s.ns));
-    }
-    dft<R, DIR>(x);
-#pragma unroll
-    for (int i = 0; i < R; ++i) v[m + M * i] = x[i];
-  }
-}
-
-// write the outputs of a stage to their Stockham positions in shared memory
-template <int E, int R>
-__device__ __forceinline__ void reg_scatter(const float2 (&v)[E], int t, int T, const Stage& s,
-                                            float2* sm) {
-  constexpr int M = E / R;
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    const int j = t + T * m;
-    const int q = div_ns(j, s);
-    const int base = q * s.ns * R + (j - q * s.ns);
-#pragma unroll
-    for (int i = 0; i < R; ++i) sm[spad(base + i * s.ns)] = v[m + M * i];
-  }
-}
-
-template <int E, int DIR>
-__device__ __forceinline__ void reg_stage_dispatch(float2 (&v)[E], int t, int T, const Stage& s,
-                                                   const float2* __restrict__ tw) {
-  switch (s.radix) {
-#define PLFFT_B200_CASE(R)                                  \
-  case R:                                                   \
-    if constexpr (E % R == 0) reg_butterflies<E, R, DIR>(v, t, T, s, tw); \
-    break;
-    PLFFT_B200_RADIX_LIST(PLFFT_B200_CASE)
-#undef PLFFT_B200_CASE
-    default:
-      break;
-  }
-}
-
-template <int E>
-__device__ __forceinline__ void reg_scatter_dispatch(const float2 (&v)[E], int t, int T, const Stage& s,
-                                                     float2* sm) {
-  switch (s.radix) {
-#define PLFFT_B200_CASE(R)                                   \
-  case R:                                                    \
-    if constexpr (E % R == 0) reg_scatter<E, R>(v, t, T, s, sm); \
-    break;
-    PLFFT_B200_RADIX_LIST(PLFFT_B200_CASE)
-#undef PLFFT_B200_CASE
-    default:
-      break;
-  }
-}
-
-struct GroupSync {
-  bool cta;  // true: __syncthreads, false: the group lives inside one warp
-  __device__ __forceinline__ void operator()() const {
-    if (cta)
-      __syncthreads();
-    else
-      __syncwarp();
-  }
-};
-
-// On entry v[q] = x[t + T*q]; on exit v[q] = X[t + T*q].
-// sm: this transform's shared-memory slice (spad_len(N) complex).
-template <int E, int DIR>
-__device__ __forceinline__ void reg_fft(float2 (&v)[E], const FftDesc& d, int t, int T, float2* sm,
-                                        const float2* __restrict__ tw, GroupSync sync) {
-  reg_stage_dispatch<E, DIR>(v, t, T, d.st[0], tw);
-  for (int s = 1; s < d.nstages; ++s) {
-    if (s > 1) sync();  // previous exchange fully read before it is overwritten
-    reg_scatter_dispatch<E>(v, t, T, d.st[s - 1], sm);
-    sync();
-#pragma unroll
-    for (int q = 0; q < E; ++q) v[q] = sm[spad(t + T * q)];
-    reg_stage_dispatch<E, DIR>(v, t, T, d.st[s], tw);
-  }
 }
 
 // ===========================================================================

@@ -1,0 +1,137 @@
+"""Mixed-radix tile engine: C2C in FP32, FP64 and FP16 and the one-pass real
+transforms, at the lengths where tiles, stages and layouts change."""
+import numpy as np
+import pytest
+
+import oracle
+import plfft
+from helpers import gather, seeded_complex, seeded_real, span, to_dev
+
+pytestmark = pytest.mark.gpu
+
+# one stage (2, 13, 16), two, three, four; primes of the radix menu; a tile of
+# many transforms and of one; the longest one- and two-buffer tiles
+LENGTHS = [2, 13, 16, 18, 121, 169, 210, 360, 1000, 1001, 1155, 2187, 4000, 6561, 8000, 12000, 14336]
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+@pytest.mark.parametrize("direction", [-1, 1])
+def test_c2c_fp32(n, direction):
+    import torch
+
+    hm = 37 if n <= 4000 else 3  # a ragged last tile
+    # unit stride with padded members, members interleaved, both sides mixed
+    for is_, id_, os_, od in [(1, n + 1, 1, n), (hm + 2, 1, hm + 2, 1), (1, n, hm, 1), (hm, 1, 2, 2 * n + 1)]:
+        x = seeded_complex(span(hm, id_, n, is_), n)
+        y = torch.full((span(hm, od, n, os_),), 7.0, dtype=torch.complex64, device="cuda")
+        plan = plfft.make_plan("c2c", n, hm, is_, id_, os_, od, direction=direction, scale=0.5)
+        plan.execute(to_dev(x).data_ptr(), y.data_ptr())
+        got = y.cpu().numpy()
+        ref = 0.5 * oracle.c2c(gather(x, hm, id_, n, is_).astype(np.complex128), direction, method="fft")
+        assert oracle.rel_l2(gather(got, hm, od, n, os_), ref) <= oracle.fp32_tol(n), plan.describe()
+        touched = np.zeros(got.size, bool)
+        touched[(np.arange(hm)[:, None] * od + np.arange(n)[None, :] * os_).ravel()] = True
+        assert np.all(got[~touched] == 7.0), "wrote outside the members"
+
+
+# n <= 4096 (one pass), one-buffer and two-buffer tiles, a two-pass length;
+# 2^-53 per rounding, 8 log2 n of them
+@pytest.mark.parametrize("n", [2, 13, 64, 143, 1000, 2048, 4096, 5000, 8192, 30000])
+@pytest.mark.parametrize("strided", [False, True])
+def test_c2c_fp64(n, strided):
+    import torch
+
+    hm = 9
+    is_, id_ = (hm + 1, 1) if strided else (1, n)
+    rng = np.random.default_rng(n)
+    m = span(hm, id_, n, is_)
+    x = rng.uniform(-1, 1, m) + 1j * rng.uniform(-1, 1, m)
+    for direction in (-1, 1):
+        plan = plfft.make_plan("c2c", n, hm, is_, id_, is_, id_, direction=direction, data_type=plfft.DataType.FP64)
+        y = torch.zeros(m, dtype=torch.complex128, device="cuda")
+        plan.execute(to_dev(x).data_ptr(), y.data_ptr())
+        xl = torch.from_numpy(gather(x, hm, id_, n, is_))
+        ref = (torch.fft.fft(xl) if direction < 0 else torch.fft.ifft(xl) * n).numpy()
+        tol = 8 * max(1.0, np.log2(n)) * 2.0**-53
+        assert oracle.rel_l2(gather(y.cpu().numpy(), hm, id_, n, is_), ref) <= tol, plan.describe()
+
+
+# binary16 buffers on 4-byte and on odd 2-byte boundaries, strided and dense:
+# one rounding of the output (2^-11) on top of FP32
+@pytest.mark.parametrize("n", [2, 16, 100, 1000, 1024, 4096])
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("strided", [False, True])
+def test_c2c_fp16(n, offset, strided):
+    import torch
+
+    hm = 21
+    s, d = (hm, 1) if strided else (1, n)
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-1, 1, 2 * n * hm + offset).astype(np.float16)
+    y = torch.zeros(x.size, dtype=torch.float16, device="cuda")
+    plan = plfft.make_plan("c2c", n, hm, s, d, s, d, data_type=plfft.DataType.FP16, scale=n**-0.5)
+    dx = to_dev(x)
+    plan.execute(dx.data_ptr() + 2 * offset, y.data_ptr() + 2 * offset)
+    z = x[offset:].astype(np.float64).view(np.complex128)
+    ref = oracle.c2c(gather(z, hm, d, n, s), -1, method="fft") * n**-0.5
+    got = y.cpu().numpy()[offset:].astype(np.float64).view(np.complex128)
+    assert oracle.rel_l2(gather(got, hm, d, n, s), ref) <= 2.0**-11 + oracle.fp32_tol(n), plan.describe()
+
+
+REAL_LENGTHS = [4, 6, 26, 32, 100, 242, 1000, 2002, 4374, 8000, 20000]
+R2R = [plfft.R2RKind.DCT_2, plfft.R2RKind.DCT_3, plfft.R2RKind.DCT_4, plfft.R2RKind.DST_2, plfft.R2RKind.DST_3,
+       plfft.R2RKind.DST_4, plfft.R2RKind.DHT, plfft.R2RKind.R2HC, plfft.R2RKind.HC2R]
+
+
+@pytest.mark.parametrize("n", REAL_LENGTHS)
+@pytest.mark.parametrize("pad", [0, 1])
+def test_r2c_c2r(n, pad):
+    import torch
+
+    hm, h = 11, n // 2 + 1
+    x = seeded_real(span(hm, n + pad, n, 1), n)
+    f = plfft.make_plan("r2c", n, hm, 1, n + pad, 1, h + pad)
+    y = torch.full((span(hm, h + pad, h, 1),), 7.0, dtype=torch.complex64, device="cuda")
+    f.execute(to_dev(x).data_ptr(), y.data_ptr())
+    xl = gather(x, hm, n + pad, n, 1).astype(np.float64)
+    spec = gather(y.cpu().numpy(), hm, h + pad, h, 1)
+    assert oracle.rel_l2(spec, np.fft.rfft(xl)) <= oracle.fp32_tol(n), f.describe()
+    b = plfft.make_plan("c2r", n, hm, 1, h + pad, 1, n + pad, scale=1.0 / n)
+    z = torch.full((x.size,), 7.0, dtype=torch.float32, device="cuda")
+    b.execute(y.data_ptr(), z.data_ptr())
+    got = z.cpu().numpy()
+    assert oracle.rel_l2(gather(got, hm, n + pad, n, 1), xl) <= 2 * oracle.fp32_tol(n), b.describe()
+    if pad:
+        assert np.all(got[np.arange(hm - 1) * (n + 1) + n] == 7.0), "wrote between the members"
+
+
+@pytest.mark.parametrize("n", [6, 26, 100, 1000, 2002])
+@pytest.mark.parametrize("kind", R2R)
+def test_r2r(n, kind):
+    import torch
+
+    hm = 7
+    for pad in (0, 1):
+        x = seeded_real(span(hm, n + pad, n, 1), n)
+        plan = plfft.make_plan("r2r", n, hm, 1, n + pad, 1, n + pad, r2r_kind=kind)
+        y = torch.zeros(x.size, dtype=torch.float32, device="cuda")
+        plan.execute(to_dev(x).data_ptr(), y.data_ptr())
+        ref = oracle.r2r(gather(x, hm, n + pad, n, 1).astype(np.float64), int(kind))
+        got = gather(y.cpu().numpy(), hm, n + pad, n, 1)
+        assert oracle.rel_l2(got, ref) <= oracle.fp32_tol(2 * n), plan.describe()
+
+
+# in-place layouts whose outputs do not lie on their own member's inputs read
+# the whole batch before the first write
+def test_r2c_in_place_dense():
+    import torch
+
+    n, hm = 1000, 5
+    h = n // 2 + 1
+    x = seeded_real(hm * n, 3)
+    buf = torch.zeros(hm * 2 * h, dtype=torch.float32, device="cuda")
+    buf[: hm * n] = to_dev(x)
+    plan = plfft.make_plan("r2c", n, hm, 1, n, 1, h, alias=plfft.IoAlias.MAY_ALIAS)
+    plan.execute(buf.data_ptr(), buf.data_ptr())
+    got = buf.cpu().numpy().view(np.complex64).reshape(hm, h)
+    assert oracle.rel_l2(got, np.fft.rfft(x.reshape(hm, n).astype(np.float64))) <= oracle.fp32_tol(n), plan.describe()
