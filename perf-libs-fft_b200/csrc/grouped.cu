@@ -19,186 +19,218 @@
 // PLFFT user would otherwise run (a plan per length, reference
 // src/plfft.cpp:427-517 and the batched plan of src/batched_1d_plan.hpp).
 #include "kernels.h"
+#include "mix.cuh"
 #include "ptx.cuh"
-#include "stockham.cuh"
 
 namespace plfft_b200 {
 
-constexpr int kGroupMaxE = 32;
-constexpr int kGroupThreads = 256;
+// The on-chip transforms run the stages of the mixed-radix engine (mix.cuh)
+// with the stage list of the task in shared memory.  512 threads at 64
+// registers, two CTAs per SM: 32 warps hide the loads of one CTA's tile
+// behind the other's arithmetic, and 72 KB of tile per CTA keep 32 four-step
+// columns of 256 (whole 256-byte segments) together.
+constexpr int kGroupThreads = 512;
 
-__device__ __forceinline__ float2 group_two_level(const TwoLevel& p, int64_t e) {
-  e %= p.n;
-  const int64_t hi = e / p.l;
-  const int64_t lo = e - hi * p.l;
-  return cmul(__ldg(p.lo + lo), __ldg(p.hi + hi));
-}
+__device__ __forceinline__ float2 group_conj(float2 v, bool on) { return on ? make_float2(v.x, -v.y) : v; }
 
-template <int DIR>
-__device__ __forceinline__ void group_fft(float2* sm, int cnt, int ld, const GroupPhase& P, int desc) {
-  smem_fft<kGroupMaxE, DIR>(sm, cnt, ld, P.descs[desc], P.tws[desc], threadIdx.x, blockDim.x);
-}
+// plain loads and stores of a tile; a backward tile is the conjugate of the
+// forward transform of the conjugated input, so one set of stages serves both
+struct GroupIo {
+  const GTask* T;
+  const float2* in;
+  float2* out;
+  bool conj;
 
-__device__ __forceinline__ void group_fft_dir(int dir, float2* sm, int cnt, int ld, const GroupPhase& P, int desc) {
-  if (dir < 0)
-    group_fft<-1>(sm, cnt, ld, P, desc);
-  else
-    group_fft<1>(sm, cnt, ld, P, desc);
-}
-
-// epilogue: store result element (c, k) of a tile
-__device__ __forceinline__ void tile_store(const GTask& T, float2* out, const float2* xin, int c, int k, float2 y,
-                                           int dir) {
-  const int64_t e = T.oe0 + int64_t(c) * T.oec + int64_t(k) * T.oek;  // logical output index
-  switch (T.post_op) {
-    case GO_TWIDDLE: {
-      const float2 w = group_two_level(T.tw2, (T.col0 + c) * int64_t(k));
-      y = dir < 0 ? cmul(y, w) : cmulc(y, w);
-      break;
+  template <int R>
+  __device__ __forceinline__ void load(int c, int j, int nb, float2 (&x)[R]) const {
+    const float2* p = in + int64_t(c) * T->icdist + int64_t(j) * T->ikstride;
+    const int64_t step = int64_t(nb) * T->ikstride;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      x[i] = group_conj(*p, conj);
+      p += step;
     }
-    case GO_SPEC:
-      y = cmul(y, T.post_tab[e]);
-      break;
-    case GO_SPEC_SAVE0:
-      if (e == 0) T.sum0[0] = y;
-      y = cmul(y, T.post_tab[e]);
-      break;
-    case GO_CHIRP:
-      if (e >= T.post_len) return;
-      y = cmul(y, T.post_tab[e]);
-      break;
-    case GO_SCATTER: {
-      const float2 x0 = xin[0];
-      out[int64_t(T.perm_out[e]) * T.okstride] = cscale(cadd(x0, y), T.scale);
-      if (e == 0) out[0] = cscale(cadd(x0, T.sum0[0]), T.scale);
-      return;
-    }
-    default:
-      break;
   }
-  out[int64_t(c) * T.ocdist + int64_t(k) * T.okstride] = T.scale == 1.f ? y : cscale(y, T.scale);
+  template <int R>
+  __device__ __forceinline__ void store(int c, int k, int kstep, float2 (&x)[R]) const {
+    float2* p = out + int64_t(c) * T->ocdist + int64_t(k) * T->okstride;
+    const int64_t step = int64_t(kstep) * T->okstride;
+    const bool tw = T->post_op == GO_TWIDDLE;
+    const float s = T->scale;
+    const uint32_t col = uint32_t(T->col0) + uint32_t(c);
+    const int shift = T->tw2_shift;
+    const float2* lo = T->tw2.lo;
+    const float2* hi = T->tw2.hi;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      float2 y = x[i];  // a backward tile's twiddle is conj(W): conj(y W) = conj(y) conj(W)
+      if (tw) {
+        const uint32_t e = col * uint32_t(k + i * kstep);
+        y = cmul(y, cmul(__ldg(lo + (e & ((1u << shift) - 1u))), __ldg(hi + (e >> shift))));
+      }
+      *p = cscale(group_conj(y, conj), s);
+      p += step;
+    }
+  }
+};
+
+// middle stages [first, last) of the tile in `src`; returns the buffer that
+// holds the result
+__device__ __forceinline__ float2* group_stages(const MixDesc& d, const float2* tw, float2* src, float2* dst,
+                                                const GroupIo& io, int cnt, int first, int last) {
+  for (int si = first; si < last; ++si) {
+    mix_dispatch<float2, -1, MIX_MID>(d, si, tw, src, dst, io, cnt);
+    __syncthreads();
+    float2* t = src;
+    src = dst;
+    dst = t;
+  }
+  return src;
 }
 
-__device__ void run_tile(const GTask& T, const GroupPhase& P, float2* sm) {
-  const int n = T.n, cnt = T.cnt;
-  const int ld = spad_len(n);
-  const int total = cnt * n;
-  const float2* in = P.bases[T.in_buf] + T.in_off;
-  float2* out = P.bases[T.out_buf] + T.out_off;
+__device__ void run_tile(const GTask& T, const MixDesc& d, const GroupPhase& P, float2* sm) {
+  const int n = T.n, cnt = T.cnt, ld = d.ld;
+  GroupIo io;
+  io.T = &T;
+  io.in = P.bases[T.in_buf] + T.in_off;
+  io.out = P.bases[T.out_buf] + T.out_off;
+  io.conj = T.dir > 0;
+  const float2* tw = P.tws[T.desc];
+  float2* src = sm;
+  float2* dst = d.inplace ? sm : sm + d.c * ld;
+  const int ns = d.nstages;
+  if (ns == 0) {  // length 1: a copy
+    for (int c = threadIdx.x; c < cnt; c += blockDim.x)
+      io.out[int64_t(c) * T.ocdist] = cscale(io.in[int64_t(c) * T.icdist], T.scale);
+    return;
+  }
+  int first = 1;
+  if (T.pre_op == GO_NONE) {
+    mix_dispatch<float2, -1, MIX_FIRST>(d, 0, tw, src, src, io, cnt);
+    __syncthreads();
+  } else {
+    // gathered or chirped inputs of a long convolution, staged in order; the
+    // convolution's forward transform, so no conjugation
+    first = 0;
+    const bool kfast = T.pre_op == GO_GATHER;
+    for (int f = threadIdx.x; f < cnt * n; f += blockDim.x) {
+      const int c = kfast ? f / n : f % cnt, k = kfast ? f - c * n : f / cnt;
+      const int64_t e = T.ie0 + int64_t(c) * T.iec + int64_t(k) * T.iek;
+      float2 v = make_float2(0.f, 0.f);
+      if (T.pre_op == GO_GATHER)
+        v = io.in[int64_t(T.perm_in[e]) * T.ikstride];
+      else if (e < T.pre_len)
+        v = cmul(io.in[int64_t(c) * T.icdist + int64_t(k) * T.ikstride], T.pre_tab[e]);
+      src[c * ld + k] = v;
+    }
+    __syncthreads();
+  }
+  if ((T.post_op == GO_NONE || T.post_op == GO_TWIDDLE) && ns > 1) {
+    float2* at = group_stages(d, tw, src, dst, io, cnt, first, ns - 1);
+    mix_dispatch<float2, -1, MIX_LAST>(d, ns - 1, tw, at, at, io, cnt);
+    return;
+  }
+  const float2* z = group_stages(d, tw, src, dst, io, cnt, first, ns);
   const float2* xin = P.bases[T.aux_buf] + T.aux_off;
-  // element f = (c, k) walks the tile with the fast index along the
-  // contiguous dimension; (c, k) is carried from one iteration to the next
-  // (one division per tile, not per element) and the loop is unrolled so
-  // that several loads are in flight per thread
-  const bool kfast_in = T.ikstride == 1 || T.pre_op == GO_GATHER;
-  {
-    const int fast = kfast_in ? n : cnt;  // extent of the fast index
-    const int bq = blockDim.x / fast, br = blockDim.x - bq * fast;
-    int slow = threadIdx.x / fast, fi = threadIdx.x - slow * fast;
-    // asynchronous copies (all of a thread's loads in flight); the chirp of
-    // a Bluestein prologue is applied in shared memory afterwards
-#pragma unroll 4
-    for (int f = threadIdx.x; f < total; f += blockDim.x) {
-      const int c = kfast_in ? slow : fi, k = kfast_in ? fi : slow;
-      float2* dst = sm + c * ld + spad(k);
-      if (T.pre_op == GO_GATHER) {
-        const int64_t e = T.ie0 + int64_t(c) * T.iec + int64_t(k) * T.iek;
-        cp_async8(dst, in + int64_t(T.perm_in[e]) * T.ikstride);
-      } else if (T.pre_op == GO_CHIRP && T.ie0 + int64_t(c) * T.iec + int64_t(k) * T.iek >= T.pre_len) {
-        *dst = make_float2(0.f, 0.f);
-      } else {
-        cp_async8(dst, in + int64_t(c) * T.icdist + int64_t(k) * T.ikstride);
+  const bool kfast = T.okstride == 1 || T.post_op == GO_SCATTER;
+  for (int f = threadIdx.x; f < cnt * n; f += blockDim.x) {
+    const int c = kfast ? f / n : f % cnt, k = kfast ? f - c * n : f / cnt;
+    float2 y = group_conj(z[c * ld + k], io.conj);
+    const int64_t e = T.oe0 + int64_t(c) * T.oec + int64_t(k) * T.oek;  // logical output index
+    switch (T.post_op) {
+      case GO_TWIDDLE: {
+        const uint32_t q = (uint32_t(T.col0) + uint32_t(c)) * uint32_t(k);
+        const float2 w = cmul(__ldg(T.tw2.lo + (q & ((1u << T.tw2_shift) - 1u))), __ldg(T.tw2.hi + (q >> T.tw2_shift)));
+        y = io.conj ? cmulc(y, w) : cmul(y, w);
+        break;
       }
-      fi += br;
-      slow += bq;
-      if (fi >= fast) {
-        fi -= fast;
-        ++slow;
+      case GO_SPEC_SAVE0:
+        if (e == 0) T.sum0[0] = y;
+        y = cmul(y, T.post_tab[e]);
+        break;
+      case GO_SPEC:
+        y = cmul(y, T.post_tab[e]);
+        break;
+      case GO_CHIRP:
+        if (e >= T.post_len) continue;
+        y = cmul(y, T.post_tab[e]);
+        break;
+      case GO_SCATTER: {
+        const float2 x0 = xin[0];
+        io.out[int64_t(T.perm_out[e]) * T.okstride] = cscale(cadd(x0, y), T.scale);
+        if (e == 0) io.out[0] = cscale(cadd(x0, T.sum0[0]), T.scale);
+        continue;
       }
+      default: break;
     }
-    cp_async_wait_all();
-    if (T.pre_op == GO_CHIRP) {
-      __syncthreads();
-      for (int f = threadIdx.x; f < total; f += blockDim.x) {
-        const int c = f / n, k = f - c * n;
-        const int64_t e = T.ie0 + int64_t(c) * T.iec + int64_t(k) * T.iek;
-        if (e < T.pre_len) sm[c * ld + spad(k)] = cmul(sm[c * ld + spad(k)], T.pre_tab[e]);
-      }
-    }
-  }
-  __syncthreads();
-  group_fft_dir(T.dir, sm, cnt, ld, P, T.desc);
-  const bool kfast_out = T.okstride == 1 || T.post_op == GO_SCATTER;
-  {
-    const int fast = kfast_out ? n : cnt;
-    const int bq = blockDim.x / fast, br = blockDim.x - bq * fast;
-    int slow = threadIdx.x / fast, fi = threadIdx.x - slow * fast;
-#pragma unroll 4
-    for (int f = threadIdx.x; f < total; f += blockDim.x) {
-      const int c = kfast_out ? slow : fi, k = kfast_out ? fi : slow;
-      tile_store(T, out, xin, c, k, sm[c * ld + spad(k)], T.dir);
-      fi += br;
-      slow += bq;
-      if (fi >= fast) {
-        fi -= fast;
-        ++slow;
-      }
-    }
+    io.out[int64_t(c) * T.ocdist + int64_t(k) * T.okstride] = cscale(y, T.scale);
   }
 }
 
-// whole Rader transform (P prime, P-1 = T.n on chip)
-__device__ void run_rader(const GTask& T, const GroupPhase& P, float2* sm) {
+// whole Rader (prime P, P - 1 = T.n on chip) or Bluestein transform (length
+// T.pre_len, convolution length T.n on chip)
+template <bool RADER>
+__device__ void run_conv(const GTask& T, const MixDesc& d, const GroupPhase& P, float2* sm) {
   const int m = T.n;
-  const int ld = spad_len(m);
-  const float2* in = P.bases[T.in_buf] + T.in_off;
-  float2* out = P.bases[T.out_buf] + T.out_off;
+  GroupIo io;
+  io.T = &T;
+  io.in = P.bases[T.in_buf] + T.in_off;
+  io.out = P.bases[T.out_buf] + T.out_off;
+  io.conj = false;
+  const float2* tw = P.tws[T.desc];
+  float2* other = d.inplace ? sm : sm + d.ld;
   __shared__ float2 a0;
-  for (int q = threadIdx.x; q < m; q += blockDim.x) sm[spad(q)] = in[int64_t(T.perm_in[q]) * T.ikstride];
+  for (int q = threadIdx.x; q < m; q += blockDim.x) {
+    float2 v = make_float2(0.f, 0.f);
+    if (RADER)
+      v = io.in[int64_t(T.perm_in[q]) * T.ikstride];
+    else if (q < T.pre_len)
+      v = cmul(io.in[int64_t(q) * T.ikstride], T.pre_tab[q]);
+    sm[q] = v;
+  }
   __syncthreads();
-  group_fft<-1>(sm, 1, ld, P, T.desc);
-  if (threadIdx.x == 0) a0 = sm[0];
+  float2* z = group_stages(d, tw, sm, other, io, 1, 0, d.nstages);
+  // the product, conjugated: the inverse transform is the conjugate of the
+  // forward one of it
+  const float2* spec = RADER ? T.post_tab : T.post_tab2;
+  for (int q = threadIdx.x; q < m; q += blockDim.x) {
+    const float2 v = z[q];
+    if (RADER && q == 0) a0 = v;
+    z[q] = group_conj(cmul(v, spec[q]), true);
+  }
   __syncthreads();
-  for (int q = threadIdx.x; q < m; q += blockDim.x) sm[spad(q)] = cmul(sm[spad(q)], T.post_tab[q]);
-  __syncthreads();
-  group_fft<1>(sm, 1, ld, P, T.desc);
-  const float2 x0 = in[0];
-  for (int q = threadIdx.x; q < m; q += blockDim.x)
-    out[int64_t(T.perm_out[q]) * T.okstride] = cscale(cadd(x0, sm[spad(q)]), T.scale);
-  if (threadIdx.x == 0) out[0] = cscale(cadd(x0, a0), T.scale);
-}
-
-// whole Bluestein transform (length T.pre_len, convolution length T.n on chip)
-__device__ void run_blue(const GTask& T, const GroupPhase& P, float2* sm) {
-  const int m = T.n, nl = T.pre_len;
-  const int ld = spad_len(m);
-  const float2* in = P.bases[T.in_buf] + T.in_off;
-  float2* out = P.bases[T.out_buf] + T.out_off;
-  for (int j = threadIdx.x; j < m; j += blockDim.x)
-    sm[spad(j)] = j < nl ? cmul(in[int64_t(j) * T.ikstride], T.pre_tab[j]) : make_float2(0.f, 0.f);
-  __syncthreads();
-  group_fft<-1>(sm, 1, ld, P, T.desc);
-  for (int k = threadIdx.x; k < m; k += blockDim.x) sm[spad(k)] = cmul(sm[spad(k)], T.post_tab2[k]);
-  __syncthreads();
-  group_fft<1>(sm, 1, ld, P, T.desc);
-  for (int k = threadIdx.x; k < nl; k += blockDim.x)
-    out[int64_t(k) * T.okstride] = cscale(cmul(sm[spad(k)], T.pre_tab[k]), T.scale);
+  z = group_stages(d, tw, z, z == sm ? other : sm, io, 1, 0, d.nstages);
+  if (RADER) {
+    const float2 x0 = io.in[0];
+    for (int q = threadIdx.x; q < m; q += blockDim.x)
+      io.out[int64_t(T.perm_out[q]) * T.okstride] = cscale(cadd(x0, group_conj(z[q], true)), T.scale);
+    if (threadIdx.x == 0) io.out[0] = cscale(cadd(x0, a0), T.scale);
+  } else {
+    for (int k = threadIdx.x; k < T.pre_len; k += blockDim.x)
+      io.out[int64_t(k) * T.okstride] = cscale(cmul(group_conj(z[k], true), T.pre_tab[k]), T.scale);
+  }
 }
 
 __global__ void __launch_bounds__(kGroupThreads, 2) grouped_kernel(const GroupPhase P) {
   extern __shared__ float2 smem[];
   __shared__ int cur;
+  __shared__ GTask T;
+  __shared__ MixDesc d;
   for (;;) {
     if (threadIdx.x == 0) cur = atomicAdd(P.counter, 1);
     __syncthreads();
     const int t = cur;
-    __syncthreads();
     if (t >= P.ntasks) break;
-    const GTask T = P.tasks[t];
+    static_assert(sizeof(GTask) % 4 == 0 && sizeof(MixDesc) % 4 == 0, "copied word by word");
+    const int* tsrc = reinterpret_cast<const int*>(P.tasks + t);
+    const int* dsrc = reinterpret_cast<const int*>(P.descs + P.tasks[t].desc);
+    for (int i = threadIdx.x; i < int(sizeof(GTask) / 4); i += blockDim.x) reinterpret_cast<int*>(&T)[i] = tsrc[i];
+    for (int i = threadIdx.x; i < int(sizeof(MixDesc) / 4); i += blockDim.x) reinterpret_cast<int*>(&d)[i] = dsrc[i];
+    __syncthreads();
     switch (T.type) {
-      case GT_TILE: run_tile(T, P, smem); break;
-      case GT_RADER: run_rader(T, P, smem); break;
-      case GT_BLUE: run_blue(T, P, smem); break;
+      case GT_TILE: run_tile(T, d, P, smem); break;
+      case GT_RADER: run_conv<true>(T, d, P, smem); break;
+      case GT_BLUE: run_conv<false>(T, d, P, smem); break;
       default: break;
     }
     __syncthreads();
@@ -214,6 +246,7 @@ __global__ void __launch_bounds__(kGroupThreads, 2) grouped_kernel(const GroupPh
   }
 }
 
+int group_threads() { return kGroupThreads; }
 int group_max_smem_elems() { return 72 * 1024 / int(sizeof(float2)); }
 
 cudaError_t launch_grouped(const GroupPhase& P, int grid, int smem_bytes, cudaStream_t st) {

@@ -23,25 +23,19 @@
 #include <cstring>
 #include <map>
 #include <sstream>
+#include <tuple>
 
 #include "../../include/plfft.h"
 #include "../../include/plfft_cuda.h"
 #include "plan.hpp"
+#include "plan_mix.hpp"
 
 namespace plfft_b200 {
 
 namespace {
 
 constexpr int kGroupOnChip = 8192;  // longest on-chip length of the grouped kernel
-constexpr int kGroupE = 32;
-constexpr int kGroupThr = 256;
 constexpr int kPhases = 4;
-
-bool tile_fits(int L, int cnt, const std::vector<int>& radices) {
-  for (int R : radices)
-    if (int64_t(cnt) * (L / R) > int64_t(kGroupE / R) * kGroupThr) return false;
-  return int64_t(cnt) * spad_len(L) <= group_max_smem_elems();
-}
 
 struct Tables {
   DevBuf perm_in, perm_out, spec, chirp;
@@ -72,9 +66,11 @@ struct GroupData {
   int64_t count = 0;
   std::vector<GTask> tasks[kPhases];
   DevBuf tasks_dev[kPhases];
-  std::vector<FftDesc> descs;
-  std::vector<std::unique_ptr<DevBuf>> tws;
-  std::map<int, int> desc_of;
+  std::vector<MixDesc> descs;
+  std::vector<std::shared_ptr<DevBuf>> tws;
+  std::map<int, MixDesc> laid;                   // stages per length (n = 0: none)
+  std::map<int, std::shared_ptr<DevBuf>> tw_of;  // twiddles per length
+  std::map<std::tuple<int, int, bool, bool>, int> desc_of;
   DevBuf descs_dev, tws_dev;
   std::map<int64_t, std::unique_ptr<Tables>> rader, blue;
   std::map<int64_t, std::unique_ptr<DevBuf>> lo, hi;  // two-level tables per length
@@ -95,29 +91,59 @@ struct GroupData {
     if (graph) cudaGraphExecDestroy(graph);
   }
 
-  int desc(int L) {
-    auto it = desc_of.find(L);
+  // the tile of cnt transforms of length L, if it fits the kernel's CTA
+  bool tile_fits(int L, int cnt, MixDesc* d = nullptr) {
+    auto it = laid.find(L);
+    if (it == laid.end()) {
+      MixDesc t;
+      if (!mix_tile_layout(t, L, std::min(shape.max_radix, 16))) t.n = 0;
+      it = laid.emplace(L, t).first;
+    }
+    if (it->second.n == 0) return false;
+    MixDesc t = it->second;
+    if (!mix_tile_set(t, cnt, group_threads(), group_max_smem_elems())) return false;
+    if (d) *d = t;
+    return true;
+  }
+
+  // index of the tile description of cnt transforms of length L; cf: the
+  // user's side is strided, consecutive lanes take consecutive transforms
+  int desc(int L, int cnt, bool cf_in, bool cf_out) {
+    const auto key = std::make_tuple(L, cnt, cf_in, cf_out);
+    auto it = desc_of.find(key);
     if (it != desc_of.end()) return it->second;
-    std::vector<float2> tw;
-    const FftDesc d = make_desc(L, factor_radices(L, shape.max_radix), tw);
-    auto buf = std::make_unique<DevBuf>();
-    if (buf->upload(tw) != cudaSuccess) return -1;
+    MixDesc d;
+    if (!tile_fits(L, cnt, &d)) return -1;
+    d.cf_in = cf_in;
+    d.cf_out = cf_out;
+    d.cf_mid = cnt >= 16;
+    std::shared_ptr<DevBuf>& buf = tw_of[L];
+    // a row of ones for stage 0, which a staged tile runs as a middle stage
+    const int ones = d.nstages ? d.st[0].radix - 1 : 0;
+    if (!buf) {
+      std::vector<float2> tw(size_t(ones), make_float2(1.f, 0.f));
+      const std::vector<float2> rest = mix_twiddle_list<float2>(d);
+      tw.insert(tw.end(), rest.begin(), rest.end());
+      buf = std::make_shared<DevBuf>();
+      if (buf->upload(tw) != cudaSuccess) return -1;
+    }
+    for (int s = 1; s < d.nstages; ++s) d.st[s].tw_off += ones;
     descs.push_back(d);
-    tws.push_back(std::move(buf));
+    tws.push_back(buf);
     const int idx = int(descs.size()) - 1;
-    desc_of[L] = idx;
+    desc_of[key] = idx;
     return idx;
   }
 
   bool onchip(int64_t L, int cnt = 1) {
     if (L > kGroupOnChip || !is_smooth(L)) return false;
-    return tile_fits(int(L), cnt, factor_radices(L, shape.max_radix));
+    return tile_fits(int(L), cnt);
   }
 
   // largest tile count that fits for length L (up to cap)
   int tile_count(int L, int cap) {
     int c = cap;
-    while (c > 1 && !tile_fits(L, c, factor_radices(L, shape.max_radix))) --c;
+    while (c > 1 && !tile_fits(L, c)) --c;
     return c;
   }
 
@@ -228,10 +254,12 @@ struct GroupData {
                      int64_t s1, const GTask& pro, const GTask& epi) {
     int64_t m1, m2;
     if (!split(m, m1, m2)) return false;
-    const int d1 = desc(int(m1)), d2 = desc(int(m2));
-    if (d1 < 0 || d2 < 0) return false;
     const TwoLevel tl = two_level(m);
+    int shift = 0;
+    while ((1 << shift) < tl.l) ++shift;
     const int c1 = tile_count(int(m1), shape.tile_cap), c2 = tile_count(int(m2), shape.tile_cap);
+    const int d1 = desc(int(m1), c1, true, true), d2 = desc(int(m2), c2, false, true);
+    if (d1 < 0 || d2 < 0) return false;
     for (int64_t col0 = 0; col0 < m2; col0 += c1) {
       GTask T = base_task(GT_TILE, tdir, int(m1), int(std::min<int64_t>(c1, m2 - col0)), d1);
       T.in_buf = in_buf;
@@ -252,6 +280,7 @@ struct GroupData {
       T.post_op = GO_TWIDDLE;
       T.col0 = col0;
       T.tw2 = tl;
+      T.tw2_shift = shift;
       tasks[pcol].push_back(T);
     }
     for (int64_t row0 = 0; row0 < m1; row0 += c2) {
@@ -344,7 +373,7 @@ struct GroupData {
                  di >= n && dout >= n)
             ++run;
         }
-        GTask T = base_task(GT_TILE, dir, int(n), run, desc(int(n)));
+        GTask T = base_task(GT_TILE, dir, int(n), run, desc(int(n), run, false, false));
         T.in_buf = 0;
         T.in_off = in_offs[i];
         T.ikstride = 1;
@@ -358,7 +387,7 @@ struct GroupData {
         i += run - 1;
       } else if (pl.kind == 1) {
         Tables* t = rader_tables(n);
-        GTask T = base_task(GT_RADER, dir, int(pl.m), 1, desc(int(pl.m)));
+        GTask T = base_task(GT_RADER, dir, int(pl.m), 1, desc(int(pl.m), 1, false, false));
         T.in_buf = 0;
         T.in_off = in_offs[i];
         T.ikstride = 1;
@@ -372,7 +401,7 @@ struct GroupData {
         ++nrader;
       } else if (pl.kind == 2) {
         Tables* t = blue_tables(n, pl.m);
-        GTask T = base_task(GT_BLUE, dir, int(pl.m), 1, desc(int(pl.m)));
+        GTask T = base_task(GT_BLUE, dir, int(pl.m), 1, desc(int(pl.m), 1, false, false));
         T.in_buf = 0;
         T.in_off = in_offs[i];
         T.ikstride = 1;
@@ -440,7 +469,14 @@ struct GroupData {
       };
       std::stable_sort(tasks[p].begin(), tasks[p].end(),
                        [&](const GTask& a, const GTask& b) { return cost(a) > cost(b); });
-      for (const GTask& t : tasks[p]) max_elems = std::max(max_elems, t.cnt * spad_len(t.n));
+      for (const GTask& t : tasks[p]) {
+        if (t.desc < 0) {
+          why = "device allocation failed";
+          return false;
+        }
+        const MixDesc& d = descs[t.desc];
+        max_elems = std::max(max_elems, d.c * d.ld * (d.inplace ? 1 : 2));
+      }
       if (!tasks[p].empty() && tasks_dev[p].upload(tasks[p]) != cudaSuccess) return false;
     }
     smem_bytes = max_elems * int(sizeof(float2));
@@ -461,7 +497,7 @@ struct GroupData {
       GroupPhase P{};
       P.tasks = tasks_dev[p].as<GTask>();
       P.ntasks = int(tasks[p].size());
-      P.descs = descs_dev.as<FftDesc>();
+      P.descs = descs_dev.as<MixDesc>();
       P.tws = tws_dev.as<const float2*>();
       P.bases[0] = const_cast<float2*>(static_cast<const float2*>(in));
       P.bases[1] = static_cast<float2*>(out);

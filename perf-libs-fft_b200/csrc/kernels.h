@@ -8,6 +8,7 @@
 #include <utility>
 #include <vector>
 
+#include "mix.h"
 #include "stockham_desc.h"
 
 namespace plfft_b200 {
@@ -205,12 +206,13 @@ struct GTask {
   const int* perm_out;
   float2* sum0;
   TwoLevel tw2;
+  int tw2_shift;  // log2 of tw2.l
   float scale;
 };
 struct GroupPhase {
   const GTask* tasks;
   int ntasks;
-  const FftDesc* descs;
+  const MixDesc* descs;  // stage 0 has a row of ones in its twiddle table
   const float2* const* tws;
   float2* bases[kGroupBuffers];
   int* counter;
@@ -219,6 +221,7 @@ struct GroupPhase {
 cudaError_t launch_grouped(const GroupPhase& P, int grid, int smem_bytes, cudaStream_t st);
 int grouped_blocks_per_sm(int smem_bytes);
 int group_max_smem_elems();
+int group_threads();
 
 // Fused single-kernel real transforms for N = 2M, M a power of two
 // (real_fused.cu).  Distances count elements of each buffer's own type.
