@@ -44,24 +44,20 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
 
-// the same helpers on double2, and the few that build or scale either type,
-// so one codelet body serves FP32 and FP64
-__device__ __forceinline__ float2 cmake(float x, float y) { return make_float2(x, y); }
-__device__ __forceinline__ double2 cmake(double x, double y) { return make_double2(x, y); }
-// s * a + b with a real s
-__device__ __forceinline__ float2 cfma(float2 a, float s, float2 b) { return __ffma2_rn(a, make_float2(s, s), b); }
-__device__ __forceinline__ double2 cfma(double2 a, double s, double2 b) {
-  return make_double2(fma(a.x, s, b.x), fma(a.y, s, b.y));
-}
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ double2 cmulc(double2 a, double2 b) {
-  return make_double2(fma(a.x, b.x, a.y * b.y), fma(a.y, b.x, -a.x * b.y));
-}
-__device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
+// Two complex FP32 numbers of two transforms side by side: (re, re) and
+// (im, im) in one packed register pair each.  Complex products, rotations by
+// i and sums of both transforms are then packed instructions on whole
+// operands, with none of the half swaps and sign copies that a packed
+// (re, im) product needs.
+struct alignas(16) cpair {
+  float2 re, im;
+};
+__device__ __forceinline__ float2 fneg2(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ float2 fdup(float s) { return make_float2(s, s); }
+__device__ __forceinline__ float2 fsub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+
+// The helpers below are what the codelets use, on each element type: float2
+// and double2 (one complex number) and cpair (two).
 template <class V>
 struct ScalarOf;
 template <>
@@ -72,17 +68,89 @@ template <>
 struct ScalarOf<double2> {
   using type = double;
 };
+template <>
+struct ScalarOf<cpair> {
+  using type = float;
+};
 template <class V>
 using scalar_of = typename ScalarOf<V>::type;
 
+template <class V>
+__device__ __forceinline__ V czero();
+template <>
+__device__ __forceinline__ float2 czero<float2>() { return make_float2(0.f, 0.f); }
+template <>
+__device__ __forceinline__ double2 czero<double2>() { return make_double2(0.0, 0.0); }
+template <>
+__device__ __forceinline__ cpair czero<cpair>() { return cpair{make_float2(0.f, 0.f), make_float2(0.f, 0.f)}; }
+__device__ __forceinline__ float2 cneg(float2 a) { return make_float2(-a.x, -a.y); }
+__device__ __forceinline__ double2 cneg(double2 a) { return make_double2(-a.x, -a.y); }
+__device__ __forceinline__ cpair cneg(cpair a) { return cpair{fneg2(a.re), fneg2(a.im)}; }
+// s * a + b with a real s
+__device__ __forceinline__ float2 cfma(float2 a, float s, float2 b) { return __ffma2_rn(a, make_float2(s, s), b); }
+__device__ __forceinline__ double2 cfma(double2 a, double s, double2 b) {
+  return make_double2(fma(a.x, s, b.x), fma(a.y, s, b.y));
+}
+__device__ __forceinline__ cpair cfma(cpair a, float s, cpair b) {
+  return cpair{__ffma2_rn(a.re, fdup(s), b.re), __ffma2_rn(a.im, fdup(s), b.im)};
+}
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ cpair cadd(cpair a, cpair b) { return cpair{__fadd2_rn(a.re, b.re), __fadd2_rn(a.im, b.im)}; }
+__device__ __forceinline__ cpair csub(cpair a, cpair b) { return cpair{fsub2(a.re, b.re), fsub2(a.im, b.im)}; }
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
+}
+__device__ __forceinline__ double2 cmulc(double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, a.y * b.y), fma(a.y, b.x, -a.x * b.y));
+}
+// both numbers of a pair times one factor w
+__device__ __forceinline__ cpair cmul(cpair a, float2 w) {
+  const float2 wr = fdup(w.x), wi = fdup(w.y);
+  return cpair{__ffma2_rn(a.im, fneg2(wi), __fmul2_rn(a.re, wr)), __ffma2_rn(a.im, wr, __fmul2_rn(a.re, wi))};
+}
+__device__ __forceinline__ cpair cmulc(cpair a, float2 w) {
+  const float2 wr = fdup(w.x), wi = fdup(w.y);
+  return cpair{__ffma2_rn(a.im, wi, __fmul2_rn(a.re, wr)), __ffma2_rn(a.re, fneg2(wi), __fmul2_rn(a.im, wr))};
+}
+__device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
+__device__ __forceinline__ cpair cscale(cpair a, float s) {
+  return cpair{__fmul2_rn(a.re, fdup(s)), __fmul2_rn(a.im, fdup(s))};
+}
+// times the constant (wr, wi)
+__device__ __forceinline__ float2 cmulk(float2 a, float wr, float wi) { return cmul(a, make_float2(wr, wi)); }
+__device__ __forceinline__ double2 cmulk(double2 a, double wr, double wi) { return cmul(a, make_double2(wr, wi)); }
+__device__ __forceinline__ cpair cmulk(cpair a, float wr, float wi) { return cmul(a, make_float2(wr, wi)); }
+
 // multiply by (s * i) where s = +1 or -1 (compile time)
+template <int S>
+__device__ __forceinline__ float2 cmul_i(float2 a) {
+  return S > 0 ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+}
+template <int S>
+__device__ __forceinline__ double2 cmul_i(double2 a) {
+  return S > 0 ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x);
+}
+template <int S>
+__device__ __forceinline__ cpair cmul_i(cpair a) {
+  return S > 0 ? cpair{fneg2(a.im), a.re} : cpair{a.im, fneg2(a.re)};
+}
+// (a + s i b, a - s i b)
 template <int S, class V>
-__device__ __forceinline__ V cmul_i(V a) {
-  return S > 0 ? cmake(-a.y, a.x) : cmake(a.y, -a.x);
+__device__ __forceinline__ void cadd_sub_i(V a, V b, V& sum, V& dif) {
+  const V t = cmul_i<S>(b);
+  sum = cadd(a, t);
+  dif = csub(a, t);
+}
+template <int S>
+__device__ __forceinline__ void cadd_sub_i(cpair a, cpair b, cpair& sum, cpair& dif) {
+  const cpair p{fsub2(a.re, b.im), __fadd2_rn(a.im, b.re)}, m{__fadd2_rn(a.re, b.im), fsub2(a.im, b.re)};
+  sum = S > 0 ? p : m;
+  dif = S > 0 ? m : p;
 }
 // twiddle multiply: DIR=-1 uses the table value w, DIR=+1 uses conj(w)
-template <int DIR, class V>
-__device__ __forceinline__ V twmul(V a, V w) {
+template <int DIR, class V, class W>
+__device__ __forceinline__ V twmul(V a, W w) {
   return DIR < 0 ? cmul(a, w) : cmulc(a, w);
 }
 
@@ -179,7 +247,7 @@ __device__ __forceinline__ void dft_odd(V* v) {
   out[0] = sum;
   SFor<1, H + 1>::run([&](auto mc) {
     constexpr int m = decltype(mc)::value;
-    V A = x0, B = cmake(S(0), S(0));
+    V A = x0, B = czero<V>();
     SFor<1, H + 1>::run([&](auto kc) {
       constexpr int k = decltype(kc)::value;
       constexpr S c = S(ce::unit_root((m * k) % R, R).c);
@@ -187,10 +255,7 @@ __device__ __forceinline__ void dft_odd(V* v) {
       A = cfma(a[k], c, A);
       B = cfma(b[k], s, B);
     });
-    // s*i*B with s = DIR
-    V iB = cmul_i<DIR>(B);
-    out[m] = cadd(A, iB);
-    out[R - m] = csub(A, iB);
+    cadd_sub_i<DIR>(A, B, out[m], out[R - m]);
   });
 #pragma unroll
   for (int k = 0; k < R; ++k) v[k] = out[k];
@@ -211,11 +276,10 @@ __device__ __forceinline__ void dft4(V* v) {
   V t0 = cadd(v[0], v[2]);
   V t1 = csub(v[0], v[2]);
   V t2 = cadd(v[1], v[3]);
-  V t3 = cmul_i<DIR>(csub(v[1], v[3]));
+  V t3 = csub(v[1], v[3]);
   v[0] = cadd(t0, t2);
   v[2] = csub(t0, t2);
-  v[1] = cadd(t1, t3);
-  v[3] = csub(t1, t3);
+  cadd_sub_i<DIR>(t1, t3, v[1], v[3]);
 }
 
 // composite radix R = R1 * R2 in registers:
@@ -243,11 +307,11 @@ __device__ __forceinline__ void dft_composite(V* v) {
       } else if constexpr (4 * e == 3 * R) {
         a[n2 * R1 + k1] = cmul_i<-DIR>(t[k1]);
       } else if constexpr (2 * e == R) {
-        a[n2 * R1 + k1] = cmake(-t[k1].x, -t[k1].y);
+        a[n2 * R1 + k1] = cneg(t[k1]);
       } else {
         constexpr S wr = S(ce::unit_root(e, R).c);
         constexpr S wi = S(DIR * ce::unit_root(e, R).s);
-        a[n2 * R1 + k1] = cmul(t[k1], cmake(wr, wi));
+        a[n2 * R1 + k1] = cmulk(t[k1], wr, wi);
       }
     });
   });

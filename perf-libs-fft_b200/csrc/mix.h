@@ -7,8 +7,14 @@
 namespace plfft_b200 {
 
 constexpr int kMixMaxStages = 8;
-// butterflies of radix R one thread holds at a time
-constexpr int mix_held(int R) { return R >= 16 ? 1 : 16 / R; }
+// Butterflies of radix R one thread holds at a time: as many as `budget`
+// elements allow, so small radices keep as many loads in flight as large
+// ones.  The budgets and launch bounds go together: FP32 pairs 12 elements
+// at 80 registers, FP64 and the grouped kernel's single FP32 numbers 16 at
+// 128 and 64.
+constexpr int mix_held(int R, int budget) { return R >= budget ? 1 : budget / R; }
+constexpr int kMixHeldPair = 12, kMixHeldSingle = 16;
+constexpr int kMixThreadsPair = 768, kMixThreads64 = 512;  // resident threads per SM, largest CTA
 
 // One radix stage of a tile of `c` transforms.  Butterfly j (< nb) of the
 // stage is q = j / ns, r = j mod ns; it reads logical elements j + i nb and
@@ -28,11 +34,11 @@ struct MixStage {
 
 struct MixDesc {
   int n, nstages;
-  int c;        // transforms per tile
-  int ld;       // shared-memory pitch of one transform, elements
+  int c;        // engine elements (FP32: pairs of transforms, FP64: transforms) per tile
+  int ld;       // shared-memory pitch of one of them, in 16-byte elements
   int nthr;     // threads per CTA
   int inplace;  // 1: one buffer, every middle stage held in registers at once; 0: two buffers
-  int cf_in, cf_mid, cf_out;  // 1: consecutive lanes take consecutive transforms, 0: consecutive butterflies
+  int cf_in, cf_mid, cf_out;  // 1: consecutive threads take consecutive elements of the tile, 0: consecutive butterflies
   uint32_t mul_c;
   MixStage st[kMixMaxStages];
 };
@@ -43,24 +49,26 @@ struct MixAddr {
 };
 
 // two-level four-step twiddle W_N^e = lo[e mod 2^shift] * hi[e >> shift]
-template <class V>
+template <class W>
 struct MixPost {
-  const V* lo;
-  const V* hi;
+  const W* lo;
+  const W* hi;
   int shift;
 };
 
-template <class V>
+// W: the twiddle type, float2 or double2
+template <class W>
 struct MixLaunch {
   const void* in;
   void* out;
   int64_t members;  // tiles = members * tpm
   int64_t ncols;    // transforms per member
-  uint32_t tpm;     // tiles per member: ceil(ncols / c)
+  uint32_t tpm;     // tiles per member
+  int wide_in, wide_out;  // FP32 pairs may be moved as aligned 16-byte words
   MixAddr ia, oa;
   double scale;
-  const V* tw;
-  MixPost<V> post;  // lo == nullptr: none
+  const W* tw;
+  MixPost<W> post;  // lo == nullptr: none
   MixDesc d;
 };
 
@@ -82,7 +90,7 @@ struct MixRealLaunch {
 bool mix_real_last_staged(int kind);
 cudaError_t launch_mix_real(int kind, const MixRealLaunch& L, cudaStream_t st);
 
-int mix_smem_bytes(const MixDesc& d, int elem_bytes);
+int mix_smem_bytes(const MixDesc& d);
 cudaError_t launch_mix_f32(int dir, const MixLaunch<float2>& L, cudaStream_t st);
 // binary16 buffers; pairs: both aligned for 4-byte (re, im) accesses
 cudaError_t launch_mix_f16(int dir, bool pairs, const MixLaunch<float2>& L, cudaStream_t st);

@@ -5,8 +5,8 @@ namespace plfft_b200 {
 
 cudaError_t launch_mix_f16(int dir, bool pairs, const MixLaunch<float2>& L, cudaStream_t st) {
   if (!pairs) return launch_mix_f16_scalar(dir, L, st);
-  return dir < 0 ? run_mix<float2, -1, MixIoC2C<float2, __half2, -1>>(L, st)
-                 : run_mix<float2, 1, MixIoC2C<float2, __half2, 1>>(L, st);
+  return dir < 0 ? run_mix<cpair, -1, MixIoPair<__half2, -1>>(L, st)
+                 : run_mix<cpair, 1, MixIoPair<__half2, 1>>(L, st);
 }
 
 }  // namespace plfft_b200

@@ -4,10 +4,10 @@
 namespace plfft_b200 {
 
 cudaError_t launch_mix_f32(int dir, const MixLaunch<float2>& L, cudaStream_t st) {
-  return dir < 0 ? run_mix<float2, -1, MixIoC2C<float2, float2, -1>>(L, st)
-                 : run_mix<float2, 1, MixIoC2C<float2, float2, 1>>(L, st);
+  return dir < 0 ? run_mix<cpair, -1, MixIoPair<float2, -1>>(L, st)
+                 : run_mix<cpair, 1, MixIoPair<float2, 1>>(L, st);
 }
 
-int mix_smem_bytes(const MixDesc& d, int elem_bytes) { return d.c * d.ld * elem_bytes * (d.inplace ? 1 : 2); }
+int mix_smem_bytes(const MixDesc& d) { return d.c * d.ld * 16 * (d.inplace ? 1 : 2); }
 
 }  // namespace plfft_b200

@@ -25,8 +25,11 @@ struct MixIoReal {
   const float2* post;  // W_N^k (DCT-IV / DST-IV: exp(i pi p / N))
   const float2* rot;   // exp(-i pi k / 2N) (DCT-IV / DST-IV: exp(i pi (4q+1) / 4N))
   int wmode, pairs_in, pairs_out;
+  int count;  // members of this tile
 
   __device__ __forceinline__ MixIoReal(const MixRealLaunch& L, int64_t col) {
+    const int64_t left = L.howmany - col;
+    count = left < 2 * L.d.c ? int(left) : 2 * L.d.c;
     m = L.d.n;
     ics = L.idist * (KIND == FR_C2R ? 2 : 1);
     ocs = L.odist * (KIND == FR_R2C ? 2 : 1);
@@ -91,15 +94,24 @@ struct MixIoReal {
       return cmul(make_float2(a, -b), __ldg(post + k));
     }
   }
+  // members 2 c and 2 c + 1 (an odd last one with a copy of itself)
   template <int R>
-  __device__ __forceinline__ void load(int c, int j, int nb, float2 (&z)[R]) const {
-    const float* x = in + int64_t(c) * ics;
+  __device__ __forceinline__ void load(int c, int j, int nb, cpair (&z)[R]) const {
+    const float* x0 = in + int64_t(2 * c) * ics;
+    const float* x1 = 2 * c + 1 < count ? x0 + ics : x0;
 #pragma unroll
-    for (int i = 0; i < R; ++i) z[i] = elem(x, j + i * nb);
+    for (int i = 0; i < R; ++i) {
+      const float2 a = elem(x0, j + i * nb), b = elem(x1, j + i * nb);
+      z[i] = cpair{make_float2(a.x, b.x), make_float2(a.y, b.y)};
+    }
   }
-  __device__ __forceinline__ void store1(int c, int k, float2 z) const {
-    float* y = out + int64_t(c) * ocs;
+  __device__ __forceinline__ void store1(int c, int k, cpair z) const {
     z = cscale(z, scale);
+    put_pair(2 * c, k, make_float2(z.re.x, z.im.x));
+    if (2 * c + 1 < count) put_pair(2 * c + 1, k, make_float2(z.re.y, z.im.y));
+  }
+  __device__ __forceinline__ void put_pair(int b, int k, float2 z) const {
+    float* y = out + int64_t(b) * ocs;
     if (pairs_out) {
       reinterpret_cast<float2*>(y)[k] = z;
     } else {
@@ -108,7 +120,7 @@ struct MixIoReal {
     }
   }
   template <int R>
-  __device__ __forceinline__ void store(int c, int k, int kstep, float2 (&z)[R]) const {
+  __device__ __forceinline__ void store(int c, int k, int kstep, cpair (&z)[R]) const {
 #pragma unroll
     for (int i = 0; i < R; ++i) store1(c, k + i * kstep, z[i]);
   }
@@ -133,91 +145,89 @@ struct MixIoReal {
       }
     }
   }
+  static __device__ __forceinline__ float2 lane(const cpair& z, int l) {
+    return l ? make_float2(z.re.y, z.im.y) : make_float2(z.re.x, z.im.x);
+  }
   // epilogue of the staged kinds: Z of the tile in natural order, pitch ld
-  __device__ __forceinline__ void finish(const float2* z, int ld, int c_tile, int cnt, uint32_t mul_half,
-                                         uint32_t mul_m) const {
+  __device__ __forceinline__ void finish(const cpair* z, int ld, int c_tile, uint32_t mul_half, uint32_t mul_m) const {
     const int n = 2 * m;
     if constexpr (KIND == FR_R2C || KIND == FR_R2HC || KIND == FR_DHT || KIND == FR_DCT2 || KIND == FR_DST2) {
       // pairs (k, M - k), k <= M / 2: V_k = e - i w o, V_{M-k} = conj(e + i w o)
       const int half = m / 2 + 1;
       for (int f = threadIdx.x; f < c_tile * half; f += blockDim.x) {
         const int c = mix_div(f, mul_half), k = f - c * half;
-        if (c >= cnt) continue;
-        const float2 zk = z[c * ld + k], zm = z[c * ld + (k ? m - k : 0)];
-        const float2 cm = make_float2(zm.x, -zm.y);
-        const float2 e = cscale(cadd(zk, cm), 0.5f);
-        const float2 o = cscale(csub(zk, cm), 0.5f);
-        const float2 wo = cmul(__ldg(post + k), o);
-        float* y = out + int64_t(c) * ocs;
-        emit(y, k, make_float2(e.x + wo.y, e.y - wo.x));
-        if (2 * k != m) emit(y, m - k, make_float2(e.x - wo.y, -(e.y + wo.x)));
+        const cpair pk = mix_ld(z + c * ld + k), pm = mix_ld(z + c * ld + (k ? m - k : 0));
+        const float2 w = __ldg(post + k);
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+          if (2 * c + l >= count) continue;
+          const float2 zk = lane(pk, l), zm = lane(pm, l);
+          const float2 cm = make_float2(zm.x, -zm.y);
+          const float2 e = cscale(cadd(zk, cm), 0.5f);
+          const float2 o = cscale(csub(zk, cm), 0.5f);
+          const float2 wo = cmul(w, o);
+          float* y = out + int64_t(2 * c + l) * ocs;
+          emit(y, k, make_float2(e.x + wo.y, e.y - wo.x));
+          if (2 * k != m) emit(y, m - k, make_float2(e.x - wo.y, -(e.y + wo.x)));
+        }
       }
     } else if constexpr (KIND == FR_DCT3 || KIND == FR_DST3) {
       // u_{2j} = Re z_j, u_{2j+1} = Im z_j; x_{2j} = u_j, x_{2j+1} = u_{N-1-j}
       for (int f = threadIdx.x; f < c_tile * m; f += blockDim.x) {
-        const int c = mix_div(f, mul_m), p = f - c * m;
-        if (c >= cnt) continue;
-        const float* u = reinterpret_cast<const float*>(z + c * ld);
-        const float a = u[p] * scale, b = u[n - 1 - p] * (KIND == FR_DST3 ? -scale : scale);
-        put2(c, p, a, b);
+        const int c = mix_div(f, mul_m), p = f - c * m, q = n - 1 - p;
+        const cpair a = mix_ld(z + c * ld + (p >> 1)), b = mix_ld(z + c * ld + (q >> 1));
+        const float2 ua = (p & 1) ? a.im : a.re, ub = (q & 1) ? b.im : b.re;  // of both members
+        const float sb = KIND == FR_DST3 ? -scale : scale;
+        if (2 * c < count) put_pair(2 * c, p, make_float2(ua.x * scale, ub.x * sb));
+        if (2 * c + 1 < count) put_pair(2 * c + 1, p, make_float2(ua.y * scale, ub.y * sb));
       }
     } else {
       // S_q = rot_q C_q: y_{2q} = 2 Re S_q, y_{N-1-2q} = +-2 Im S_q, written
       // as the pairs (y_{2p}, y_{2p+1}), the second from q = M - 1 - p
       for (int f = threadIdx.x; f < c_tile * m; f += blockDim.x) {
         const int c = mix_div(f, mul_m), p = f - c * m, q = m - 1 - p;
-        if (c >= cnt) continue;
-        const float2 a = cmul(__ldg(rot + p), z[c * ld + p]);
-        const float2 b = cmul(__ldg(rot + q), z[c * ld + q]);
-        put2(c, p, 2.f * a.x * scale, (KIND == FR_DST4 ? -2.f : 2.f) * b.y * scale);
+        const cpair a = cmul(mix_ld(z + c * ld + p), __ldg(rot + p));
+        const cpair b = cmul(mix_ld(z + c * ld + q), __ldg(rot + q));
+        const float sa = 2.f * scale, sb = KIND == FR_DST4 ? -2.f * scale : 2.f * scale;
+        if (2 * c < count) put_pair(2 * c, p, make_float2(a.re.x * sa, b.im.x * sb));
+        if (2 * c + 1 < count) put_pair(2 * c + 1, p, make_float2(a.re.y * sa, b.im.y * sb));
       }
-    }
-  }
-  __device__ __forceinline__ void put2(int c, int p, float a, float b) const {
-    float* y = out + int64_t(c) * ocs;
-    if (pairs_out) {
-      reinterpret_cast<float2*>(y)[p] = make_float2(a, b);
-    } else {
-      y[2 * p] = a;
-      y[2 * p + 1] = b;
     }
   }
 };
 
 template <int KIND>
-__global__ void __launch_bounds__(MixBounds<float2>::threads, 1)
+__global__ void __launch_bounds__(kMixThreadsPair, 1)
     mix_real_kernel(const __grid_constant__ MixRealLaunch L) {
   constexpr int DIR = mix_real_backward(KIND) ? 1 : -1;
   extern __shared__ __align__(16) unsigned char mix_smem[];
   griddep_wait();  // launched programmatically (launch_pdl.cuh)
   griddep_launch_dependents();
   const MixDesc& d = L.d;
-  float2* src = reinterpret_cast<float2*>(mix_smem);
-  float2* dst = d.inplace ? src : src + d.c * d.ld;
-  const int64_t col = int64_t(blockIdx.x) * d.c;
-  const int64_t left = L.howmany - col;
-  const int cnt = left < d.c ? int(left) : d.c;
-  const MixIoReal<KIND> io(L, col);
-  mix_dispatch<float2, DIR, MIX_FIRST>(d, 0, L.tw, src, src, io, cnt);
+  cpair* src = reinterpret_cast<cpair*>(mix_smem);
+  cpair* dst = d.inplace ? src : src + d.c * d.ld;
+  const MixIoReal<KIND> io(L, int64_t(blockIdx.x) * (2 * d.c));
+  const int cnt = (io.count + 1) / 2;
+  mix_dispatch<cpair, DIR, MIX_FIRST>(d, 0, L.tw, src, src, io, cnt);
   __syncthreads();
   const int ns = d.nstages;
   const int mid = mix_real_staged(KIND) ? ns : ns - 1;
   for (int si = 1; si < mid; ++si) {
-    mix_dispatch<float2, DIR, MIX_MID>(d, si, L.tw, src, dst, io, cnt);
+    mix_dispatch<cpair, DIR, MIX_MID>(d, si, L.tw, src, dst, io, cnt);
     __syncthreads();
-    float2* t = src;
+    cpair* t = src;
     src = dst;
     dst = t;
   }
   if constexpr (mix_real_staged(KIND)) {
-    io.finish(src, d.ld, d.c, cnt, L.mul_half, L.mul_m);
+    io.finish(src, d.ld, cnt, L.mul_half, L.mul_m);
   } else if (ns == 1) {
     for (int f = threadIdx.x; f < d.c * d.n; f += blockDim.x) {
       const int c = mix_div(f, L.mul_m), k = f - c * d.n;
       if (c < cnt) io.store1(c, k, src[c * d.ld + k]);
     }
   } else {
-    mix_dispatch<float2, DIR, MIX_LAST>(d, ns - 1, L.tw, src, dst, io, cnt);
+    mix_dispatch<cpair, DIR, MIX_LAST>(d, ns - 1, L.tw, src, dst, io, cnt);
   }
 }
 
@@ -225,10 +235,10 @@ template <int KIND>
 cudaError_t run_mix_real(const MixRealLaunch& L, cudaStream_t st) {
   auto* k = mix_real_kernel<KIND>;
   if (L.howmany <= 0) return cudaSuccess;
-  const int smem = mix_smem_bytes(L.d, int(sizeof(float2)));
+  const int smem = mix_smem_bytes(L.d);
   const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(k), smem);
   if (e != cudaSuccess) return e;
-  const int64_t grid = (L.howmany + L.d.c - 1) / L.d.c;
+  const int64_t grid = (L.howmany + 2 * L.d.c - 1) / (2 * L.d.c);
   if (grid > 0x7fffffff) return cudaErrorInvalidValue;
   return launch_pdl(k, dim3(unsigned(grid)), dim3(L.d.nthr), size_t(smem), st, L);
 }

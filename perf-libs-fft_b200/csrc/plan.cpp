@@ -349,12 +349,14 @@ struct C2CFourStepNode : Node {
         a.in = x + m0 * lay.idist;
         a.out = s;
         a.members = cnt;
+        mix_wide(a);
         cudaError_t e = launch_mix_f32(dir, a, st);
         if (e != cudaSuccess) return e;
         MixLaunch<float2> b = m2;
         b.in = s;
         b.out = y + m0 * lay.odist;
         b.members = cnt;
+        mix_wide(b);
         e = launch_mix_f32(dir, b, st);
         if (e != cudaSuccess) return e;
         continue;
@@ -637,8 +639,8 @@ static std::unique_ptr<Node> make_four_step(int64_t n, const Layout& lay, int di
   Addr ia2{n, n2, 1, n1};
   Addr oa2{lay.odist, lay.ostride, n1 * lay.ostride, n1};
   node->dir = dir;
-  const bool mix = mix_shape(node->m1.d, n1, n2, true, true, int(sizeof(float2)), false) &&
-                   mix_shape(node->m2.d, n2, n1, false, true, int(sizeof(float2)), false) &&
+  const bool mix = mix_shape(node->m1.d, n1, n2, true, true, 2, false) &&
+                   mix_shape(node->m2.d, n2, n1, false, true, 2, false) &&
                    n < (int64_t(1) << 32);  // the twiddle exponent col * k is 32 bits wide
   if (!mix) {
     node->p1 = make_tile(n1, 0, ia1, oa1, dir, 1.0f, true, why);
@@ -660,7 +662,7 @@ static std::unique_ptr<Node> make_four_step(int64_t n, const Layout& lay, int di
   }
   auto pass = [&](MixLaunch<float2>& m, DevBuf& tw, const Addr& ia, const Addr& oa, double sc) {
     m.ncols = ia.ncols;
-    m.tpm = uint32_t((ia.ncols + m.d.c - 1) / m.d.c);
+    m.tpm = uint32_t((ia.ncols + 2 * m.d.c - 1) / (2 * m.d.c));
     m.ia = MixAddr{ia.mdist, ia.cdist, ia.kstride};
     m.oa = MixAddr{oa.mdist, oa.cdist, oa.kstride};
     m.scale = sc;

@@ -137,8 +137,8 @@ std::unique_ptr<Node> make_fp64_c2c(int64_t n, const Layout& lay, int dir, doubl
   node->chunk = std::max<int64_t>(1, std::min<int64_t>(lay.howmany, (int64_t(256) << 20) / (n * 16)));
   // pass 1: columns (member, n2 index) of length n1, times W_n^{col k};
   // pass 2: rows (member, n1 index) of length n2, written transposed
-  if (!mix_shape(node->p1.d, n1, n2, true, true, int(sizeof(double2)), false) ||
-      !mix_shape(node->p2.d, n2, n1, false, true, int(sizeof(double2)), false) ||
+  if (!mix_shape(node->p1.d, n1, n2, true, true, 1, false) ||
+      !mix_shape(node->p2.d, n2, n1, false, true, 1, false) ||
       node->tw1.upload(mix_twiddle_list<double2>(node->p1.d)) != cudaSuccess ||
       node->tw2.upload(mix_twiddle_list<double2>(node->p2.d)) != cudaSuccess)
     return nullptr;

@@ -43,13 +43,13 @@ void search(int64_t n, int last, int cap, std::vector<int>& cur, double cost, st
 uint32_t magic(int d) { return d <= 1 ? 0u : uint32_t(((uint64_t(1) << 32) + uint64_t(d) - 1) / uint64_t(d)); }
 
 // bank conflicts of one warp-wide access pattern: extra passes beyond the
-// fewest, `eb`-byte elements at addr(lane), 32 banks of 4 bytes
+// fewest, `eb`-byte elements (8 or 16) at addr(lane)
 template <class F>
 int conflicts(int eb, F addr) {
   const int lanes = 128 / eb;  // lanes served per pass
   int worst = 0;
   for (int base = 0; base < 32; base += lanes) {
-    int count[32] = {0};
+    int count[16] = {0};
     int seen[32];
     int ns = 0;
     for (int l = base; l < base + lanes; ++l) {
@@ -59,10 +59,10 @@ int conflicts(int eb, F addr) {
       for (int k = 0; k < ns; ++k) dup = dup || seen[k] == a;
       if (dup) continue;
       seen[ns++] = a;
-      ++count[(a * (eb / 4)) % 32];
+      ++count[a % lanes];
     }
     int mx = 1;
-    for (int b = 0; b < 32; ++b) mx = std::max(mx, count[b]);
+    for (int b = 0; b < lanes; ++b) mx = std::max(mx, count[b]);
     worst += mx - 1;
   }
   return worst;
@@ -77,7 +77,7 @@ std::vector<int> mix_radices(int64_t n, int max_radix) {
   return best;
 }
 
-static bool mix_layout(MixDesc& d, const std::vector<int>& radices, int elem_bytes) {
+static bool mix_layout(MixDesc& d, const std::vector<int>& radices, int elem_bytes = 16) {
   const int n = d.n;
   d.nstages = int(radices.size());
   if (d.nstages < 1 || d.nstages > kMixMaxStages) return false;
@@ -102,9 +102,8 @@ static bool mix_layout(MixDesc& d, const std::vector<int>& radices, int elem_byt
     MixStage& r = d.st[s + 1];
     const int block = w.ns * w.radix;
     int best_pad = 0, best_c = -1;
-    const int pads[] = {0, 1, 2, 3, 4, 5, 8};
-    for (int pad : pads) {
-      if (pad > 0 && pad * 4 > block + 4) break;
+    for (int pad = 0; pad < 128 / elem_bytes; ++pad) {
+      if (pad > 1 && pad * 4 > block) break;  // a quarter more shared memory at most
       int c = 0;
       for (int w0 = 0; w0 < 4; ++w0) {
         const int j0 = w0 * 32 * 3;
@@ -147,23 +146,22 @@ namespace {
 
 // shared memory of an SM that tiles may fill, and of one CTA
 constexpr int kSmemPerSm = 227 * 1024, kSmemPerCta = 224 * 1024;
-// resident threads an SM has registers for: 64 per thread (FP32), 128 (FP64)
-constexpr int resident_threads(int elem_bytes) { return elem_bytes == 16 ? 512 : 1024; }
-
 // Estimated time of a shape per element, in issued instructions: every
 // stage's issue work with idle warps' share, spread over the resident
 // threads that hide its latency.
-double shape_cost(const MixDesc& d, int64_t ncols, int elem_bytes) {
-  const int64_t bytes = int64_t(d.c) * d.ld * elem_bytes * (d.inplace ? 1 : 2);
+double shape_cost(const MixDesc& d, int64_t ncols, int lanes) {
+  const int resident = lanes == 2 ? kMixThreadsPair : kMixThreads64;
+  const int held = lanes == 2 ? kMixHeldPair : kMixHeldSingle;
+  const int64_t bytes = int64_t(d.c) * d.ld * 16 * (d.inplace ? 1 : 2);
   if (bytes > kSmemPerCta) return -1;
-  const int per_sm = int(std::min<int64_t>({int64_t(resident_threads(elem_bytes) / d.nthr),
-                                            int64_t(kSmemPerSm) / (bytes + 1024), 32}));
+  const int per_sm =
+      int(std::min<int64_t>({int64_t(resident / d.nthr), int64_t(kSmemPerSm) / (bytes + 1024), 32}));
   if (per_sm < 1) return -1;
   double work = 0;
   const int warps = d.nthr / 32;
   for (int s = 0; s < d.nstages; ++s) {
     const MixStage& st = d.st[s];
-    const int nb = mix_held(st.radix);
+    const int nb = mix_held(st.radix, held);
     const int64_t per_iter = int64_t(nb) * d.nthr;
     const int64_t iters = (st.total + per_iter - 1) / per_iter;
     // butterflies issued (whole warps), plus the idle ones' index work
@@ -174,21 +172,25 @@ double shape_cost(const MixDesc& d, int64_t ncols, int elem_bytes) {
   const int64_t tiles = (ncols + d.c - 1) / d.c;
   const double used = double(ncols) / double(tiles * d.c);  // a ragged last tile
   double cost = work * 32.0 / (double(d.c) * d.n * used);
-  // fewer resident warps, or a single resident CTA (its barriers stop the
-  // whole SM), leave latency exposed
-  const double full = double(resident_threads(elem_bytes));
-  cost *= 1.0 + 0.5 * (1.0 - std::min(1.0, per_sm * d.nthr / full)) + 0.6 / per_sm;
+  // fewer resident warps, or few resident CTAs (their barriers stop a large
+  // share of the SM), leave latency exposed: N=1000 x 16384 FP32 61.9 us with
+  // six CTAs of 128 threads, 65.5 with three of 256, 96 with one of 416
+  cost *= 1.0 + 0.5 * (1.0 - std::min(1.0, per_sm * d.nthr / double(resident))) + 1.0 / per_sm;
+  // a second buffer takes shared memory from the L1 that serves the twiddles
+  // (N=500 x 32768: 59.5 us with one buffer, 71 with two)
+  if (!d.inplace) cost *= 1.12;
   // too few tiles for the chip: the tile's own latency counts
   const double waves = double(tiles) / (148.0 * per_sm);
-  if (waves < 1.0) cost *= 1.0 + 0.15 * double(d.c) * d.n / (16.0 * d.nthr);
+  if (waves < 1.0) cost *= 1.0 + 0.15 * (1.0 - waves) * double(d.c) * d.n / (16.0 * d.nthr);
   return cost;
 }
 
 }  // namespace
 
-bool mix_shape(MixDesc& d, int64_t n, int64_t ncols, bool cf_in, bool cf_out, int elem_bytes, bool staged, int c_req) {
-  const bool f64 = elem_bytes == 16;
-  const int max_thr = f64 ? 512 : 1024;
+bool mix_shape(MixDesc& d, int64_t n, int64_t count, bool cf_in, bool cf_out, int lanes, bool staged, int c_req) {
+  const int64_t ncols = (count + lanes - 1) / lanes;
+  const int max_thr = lanes == 2 ? kMixThreadsPair : kMixThreads64;
+  const int held = lanes == 2 ? kMixHeldPair : kMixHeldSingle;
   if (n < 2 || n > 16384) return false;
   const std::vector<int> radices = mix_radices(n, 16);
   if (radices.empty()) return false;
@@ -196,29 +198,29 @@ bool mix_shape(MixDesc& d, int64_t n, int64_t ncols, bool cf_in, bool cf_out, in
   double best_cost = -1;
   // strided batches move segments of c consecutive elements: whole 32-byte
   // sectors at least, 64 or 128 bytes where the tile fits
-  const int seg = (cf_in || cf_out) ? (f64 ? 4 : 8) : 1;
+  const int seg = (cf_in || cf_out) ? 4 : 1;
   const int cs[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 14, 16, 20, 24, 28, 32, 40, 48, 56, 64, 80, 96, 112, 128, 160, 192, 224, 256};
   MixDesc laid{};
   laid.n = int(n);
   laid.cf_in = cf_in;
   laid.cf_out = cf_out;
-  if (!mix_layout(laid, radices, elem_bytes)) return false;
+  if (!mix_layout(laid, radices)) return false;
   for (int c : cs) {
-    if (c_req > 0 ? c != c_req : (c > 1 && int64_t(c) * n > 8192)) continue;
+    if (c_req > 0 ? c != c_req : (c > 1 && int64_t(c) * n > 4096)) continue;
     if (c > ncols) break;
     MixDesc t = laid;
     mix_set_tile(t, c);
-    for (int thr = 32; thr <= max_thr; thr += thr < 128 ? 32 : 64) {
+    for (int thr = 32; thr <= max_thr; thr += 32) {
       int need = 0;  // threads that hold every middle stage at once
       for (int s = 1; s < t.nstages - (staged ? 0 : 1); ++s) {
-        const int nb = mix_held(t.st[s].radix);
+        const int nb = mix_held(t.st[s].radix, held);
         need = std::max(need, (t.st[s].total + nb - 1) / nb);
       }
       for (int ip = 0; ip < 2; ++ip) {
         if (ip ? need > thr : (t.nstages == 2 && !staged)) continue;
         t.nthr = thr;
         t.inplace = ip;  // two stages: one exchange, one buffer
-        double cost = shape_cost(t, ncols, elem_bytes);
+        double cost = shape_cost(t, ncols, lanes);
         if (cost < 0) continue;
         if (seg > 1 && c < seg) cost *= 1.0 + 0.35 * (double(seg) / c - 1.0);
         if (best_cost < 0 || cost < best_cost) {
@@ -248,7 +250,7 @@ bool mix_tile_set(MixDesc& d, int c, int threads, int max_elems) {
   mix_set_tile(d, c);
   bool held = true;  // every stage may run as a middle stage here
   for (int s = 0; s < d.nstages; ++s)
-    held = held && d.st[s].total <= int64_t(mix_held(d.st[s].radix)) * threads;
+    held = held && d.st[s].total <= int64_t(mix_held(d.st[s].radix, kMixHeldSingle)) * threads;
   d.inplace = held;
   return int64_t(c) * d.ld * (held ? 1 : 2) <= max_elems;
 }
@@ -287,6 +289,15 @@ std::vector<V> mix_twiddle_list(const MixDesc& d) {
 template std::vector<float2> mix_twiddle_list<float2>(const MixDesc&);
 template std::vector<double2> mix_twiddle_list<double2>(const MixDesc&);
 
+void mix_wide(MixLaunch<float2>& L) {
+  auto ok = [](const void* p, const MixAddr& a) {
+    return reinterpret_cast<uintptr_t>(p) % 16 == 0 && a.cdist == 1 && a.kstride % 2 == 0 && a.mdist % 2 == 0;
+  };
+  L.wide_in = ok(L.in, L.ia);
+  L.wide_out = ok(L.out, L.oa);
+}
+void mix_wide(MixLaunch<double2>&) {}
+
 std::string mix_describe(const MixDesc& d) {
   std::ostringstream o;
   o << "mix n=" << d.n << " c=" << d.c << " threads=" << d.nthr << (d.inplace ? " one-buffer" : " two-buffers")
@@ -307,6 +318,7 @@ struct MixNode : Node {
     MixLaunch<V> L = base;
     L.in = in;
     L.out = out;
+    mix_wide(L);
     if constexpr (sizeof(V) == 16)
       return launch_mix_f64(dir, L, st);
     else
@@ -330,8 +342,8 @@ std::unique_ptr<Node> make_mix_c2c(int64_t n, const Layout& lay, int dir, double
   int creq = 0;
   if (const char* v = std::getenv("PLFFT_B200_MIX_C")) creq = std::max(0, std::atoi(v));
   MixDesc& d = node->base.d;
-  if (!mix_shape(d, n, lay.howmany, cf_in, cf_out, int(sizeof(V)), false, creq) &&
-      !(creq && mix_shape(d, n, lay.howmany, cf_in, cf_out, int(sizeof(V)), false)))
+  if (!mix_shape(d, n, lay.howmany, cf_in, cf_out, sizeof(V) == 16 ? 1 : 2, false, creq) &&
+      !(creq && mix_shape(d, n, lay.howmany, cf_in, cf_out, sizeof(V) == 16 ? 1 : 2, false)))
     return nullptr;
   if (node->tw.upload(mix_twiddle_list<V>(d)) != cudaSuccess) {
     if (why) *why = "device allocation failed";
@@ -341,7 +353,8 @@ std::unique_ptr<Node> make_mix_c2c(int64_t n, const Layout& lay, int dir, double
   node->half = half;
   node->base.members = 1;
   node->base.ncols = lay.howmany;
-  node->base.tpm = uint32_t((lay.howmany + d.c - 1) / d.c);
+  const int64_t per_tile = int64_t(d.c) * (sizeof(V) == 16 ? 1 : 2);
+  node->base.tpm = uint32_t((lay.howmany + per_tile - 1) / per_tile);
   node->base.ia = MixAddr{0, lay.idist, lay.istride};
   node->base.oa = MixAddr{0, lay.odist, lay.ostride};
   node->base.scale = scale;
@@ -381,7 +394,7 @@ std::unique_ptr<Node> make_mix_real(int kind, int64_t n, const Layout& lay, floa
   const int64_t m = n / 2;
   auto node = std::make_unique<MixRealNode>();
   MixDesc& d = node->base.d;
-  if (!mix_shape(d, m, lay.howmany, false, false, int(sizeof(float2)), mix_real_last_staged(kind))) return nullptr;
+  if (!mix_shape(d, m, lay.howmany, false, false, 2, mix_real_last_staged(kind))) return nullptr;
   std::vector<float2> tab = mix_twiddle_list<float2>(d);
   const bool iv = kind == FR_DCT4 || kind == FR_DST4;
   const size_t post_off = tab.size();

@@ -12,20 +12,24 @@ namespace plfft_b200 {
 // radices 2..16 whose product is n, cheapest stage list first found; empty
 // if n has a prime factor above 13
 std::vector<int> mix_radices(int64_t n, int max_radix);
-// radices, tile width, threads and buffers for length n and `ncols`
-// transforms; c_req > 0 asks for a tile width.  False: not on chip.
+// radices, tile width, threads and buffers for length n and `count`
+// transforms, `lanes` of them per engine element (FP32 2, FP64 1); c_req > 0
+// asks for a tile width.  False: not on chip.
 // staged: the last stage's results go to shared memory, not to the user's
 // buffer.
-bool mix_shape(MixDesc& d, int64_t n, int64_t ncols, bool cf_in, bool cf_out, int elem_bytes, bool staged,
+bool mix_shape(MixDesc& d, int64_t n, int64_t count, bool cf_in, bool cf_out, int lanes, bool staged,
                int c_req = 0);
 // stages and pads of length n (1: no stage), then a tile of exactly c such
 // transforms for a CTA of `threads` threads and a shared-memory budget of
-// max_elems complex FP32, any stage of which may run from shared memory to
+// max_elems 16-byte elements, any stage of which may run from shared memory to
 // shared memory (false: does not fit)
 bool mix_tile_layout(MixDesc& d, int n, int max_radix);
 bool mix_tile_set(MixDesc& d, int c, int threads, int max_elems);
 template <class V>
 std::vector<V> mix_twiddle_list(const MixDesc& d);
+// sets wide_in / wide_out from the buffers and addresses
+void mix_wide(MixLaunch<float2>& L);
+void mix_wide(MixLaunch<double2>& L);
 std::string mix_describe(const MixDesc& d);
 
 // one-pass C2C of a strided batch (half: binary16 buffers, V = float2);
