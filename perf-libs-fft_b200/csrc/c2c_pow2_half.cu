@@ -1,0 +1,79 @@
+// Power-of-two C2C on binary16 data, FP32 arithmetic: the compile-time stage
+// list of pow2_stages.cuh between 4-byte (re, im) loads and stores of the
+// user's buffers, one launch and 8 bytes of HBM traffic per element.
+//
+// T = N/E threads per transform, whole warps' worth of transforms per CTA.
+// Bound by latency like its FP32 sibling, at half the bytes.  Forward and back,
+// N=1024 x 4096 each: see the figure at the dispatch in plan_mix.cpp.
+#include "kernels.h"
+#include "launch_pdl.cuh"
+#include "pow2_stages.cuh"
+#include "ptx.cuh"
+
+#include <cuda_fp16.h>
+
+namespace plfft_b200 {
+
+template <int N, int E, int DIR>
+__global__ void __launch_bounds__(pow2_max_threads<E>(), pow2_min_blocks<E>())
+    c2c_pow2_half_kernel(const Pow2HalfLaunch L) {
+  griddep_wait();  // launched programmatically (launch_pdl.cuh)
+  griddep_launch_dependents();
+  using P = P2<N, E>;
+  constexpr int T = P::T;
+  constexpr int PITCH = (spad_len_c(N) + 1) & ~1;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int grp = threadIdx.x / T, t = threadIdx.x - grp * T;
+  const int64_t b = int64_t(blockIdx.x) * L.g + grp;
+  const bool live = b < L.howmany;
+  float2* buf = reinterpret_cast<float2*>(smraw) + grp * PITCH;
+  auto sync = [&]() {
+    if constexpr (T <= 32)
+      __syncwarp();
+    else
+      __syncthreads();
+  };
+  const __half2* src = static_cast<const __half2*>(L.in) + (live ? b * L.idist : 0);
+  __half2 h[E];
+#pragma unroll
+  for (int q = 0; q < E; ++q) h[q] = live ? src[t + T * q] : __half2half2(__ushort_as_half(0));
+  float2 v[E];
+#pragma unroll
+  for (int q = 0; q < E; ++q) v[q] = __half22float2(h[q]);
+  st_bfly<T, E, P::radix(0), 1, 0, DIR>(v, t, L.tw);
+  Stages<N, E, DIR, 1>::run(v, t, buf, L.tw, sync);
+  if (!live) return;
+  __half2* dst = static_cast<__half2*>(L.out) + b * L.odist;
+#pragma unroll
+  for (int q = 0; q < E; ++q) dst[t + T * q] = __float22half2_rn(cscale(v[q], L.scale));
+}
+
+template <int N, int E>
+static cudaError_t run_half(int dir, Pow2HalfLaunch L, cudaStream_t st) {
+  constexpr int T = N / E;
+  L.g = T >= 128 ? 1 : 128 / T;
+  const int smem = L.g * ((spad_len_c(N) + 1) & ~1) * int(sizeof(float2));
+  auto k = dir < 0 ? c2c_pow2_half_kernel<N, E, -1> : c2c_pow2_half_kernel<N, E, 1>;
+  const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(k), smem);
+  if (e != cudaSuccess) return e;
+  const int64_t grid = (L.howmany + L.g - 1) / L.g;
+  return launch_pdl(k, dim3(unsigned(grid)), dim3(T * L.g), size_t(smem), st, L);
+}
+
+int pow2_half_e(int64_t n) { return n == 64 ? 8 : n == 1024 || n == 2048 || n == 8192 ? 32 : 16; }
+
+cudaError_t launch_c2c_pow2_half(int n, int dir, const Pow2HalfLaunch& L, cudaStream_t st) {
+  switch (n) {
+    case 64: return run_half<64, 8>(dir, L, st);
+    case 128: return run_half<128, 16>(dir, L, st);
+    case 256: return run_half<256, 16>(dir, L, st);
+    case 512: return run_half<512, 16>(dir, L, st);
+    case 1024: return run_half<1024, 32>(dir, L, st);
+    case 2048: return run_half<2048, 32>(dir, L, st);
+    case 4096: return run_half<4096, 16>(dir, L, st);
+    case 8192: return run_half<8192, 32>(dir, L, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+}  // namespace plfft_b200

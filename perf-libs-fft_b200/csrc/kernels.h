@@ -340,6 +340,20 @@ int fourstep_cluster_smem();
 int fourstep_cluster_capacity();
 cudaError_t launch_fourstep_cluster(int dir, const FourStepClusterLaunch& L, int max_clusters, cudaStream_t st);
 
+// Power-of-two C2C of binary16 (re, im) pairs, 64 <= n <= 8192, unit stride,
+// 4-byte aligned buffers (c2c_pow2_half.cu); the stage list has radix
+// pow2_half_e(n) stages after a leftover one
+struct Pow2HalfLaunch {
+  const void* in;
+  void* out;
+  int64_t howmany, idist, odist;
+  int g;
+  float scale;
+  const float2* tw;
+};
+int pow2_half_e(int64_t n);
+cudaError_t launch_c2c_pow2_half(int n, int dir, const Pow2HalfLaunch& L, cudaStream_t st);
+
 // FP16 data type (half_io.cu): strided binary16 <-> dense FP32 chunk;
 // comps = 1 (real) or 2 (complex) scalars per element.
 cudaError_t launch_half_gather(const void* src, float* dense, int64_t m0, int64_t cnt, int64_t n, int64_t stride,

@@ -171,11 +171,7 @@ struct HalfIoNode : Node {
   }
 };
 
-static std::unique_ptr<Node> make_half_node(const ConfigData& c, const Layout& lay, std::string* why) {
-  // C2C of an on-chip smooth length: binary16 loads and stores in the
-  // transform itself (one launch, 8 bytes per element instead of 40)
-  if (c.kind == TKind::C2C && member_in_place(c, lay))
-    if (auto t = make_mix_c2c<float2>(c.n, lay, c.payload, c.scale, true, why)) return t;
+static std::unique_ptr<Node> make_half_chunked(const ConfigData& c, const Layout& lay, std::string* why) {
   int64_t nin = 0, nout = 0;
   bool ic = false, oc = false;
   io_counts(c, nin, nout, ic, oc);
@@ -199,6 +195,15 @@ static std::unique_ptr<Node> make_half_node(const ConfigData& c, const Layout& l
   if (tail != node->chunk) node->inner_tail = make_root(c32, Layout{tail, 1, nin, 1, nout}, false, why, &note);
   if (!node->inner || (tail != node->chunk && !node->inner_tail)) return nullptr;
   return node;
+}
+
+static std::unique_ptr<Node> make_half_node(const ConfigData& c, const Layout& lay, std::string* why) {
+  // C2C of an on-chip length: binary16 loads and stores in the transform
+  // itself (one launch, 8 bytes per element instead of 40)
+  if (c.kind == TKind::C2C && member_in_place(c, lay))
+    if (auto t = make_half_c2c(c.n, lay, c.payload, c.scale, [&] { return make_half_chunked(c, lay, why); }, why))
+      return t;
+  return make_half_chunked(c, lay, why);
 }
 
 plfft_status_t build_plan(PlanData& p, std::string* why) {
