@@ -178,6 +178,13 @@ bool conv_fused_supported(int m, int e, int minb);
 int conv_fused_smem_bytes(int m, int g);
 cudaError_t launch_conv_fused(int m, int e, int minb, bool rader, const ConvFusedLaunch& L, cudaStream_t st);
 
+// The same over convolution lengths between the powers of two
+// (conv_list.cu): the radices (R0, A, B) of the shortest listed length >=
+// at_least (empty: none), and the launch for their product m.  tw: the rows of
+// A after R0 and of B after R0 A, then of B after A and of R0 after A B.
+std::vector<int> conv_list_radices(int64_t at_least);
+cudaError_t launch_conv_list(int m, bool rader, const ConvFusedLaunch& L, cudaStream_t st);
+
 // Grouped mixed-length execution (grouped.cu)
 enum GTaskType { GT_TILE = 0, GT_RADER = 1, GT_BLUE = 2 };
 enum GOp {

@@ -229,6 +229,7 @@ struct ConvFusedNode : Node {
   Layout lay{};
   float scale = 1.f;
   int e = 16, minb = 3, g = 1;
+  bool list = false;  // conv_list kernel (e, minb, g unused)
   DevBuf tw, chirp, spec, pin, pout;
   cudaError_t run(const void* in, void* out, void*, cudaStream_t st) const override {
     ConvFusedLaunch L{};
@@ -247,11 +248,17 @@ struct ConvFusedNode : Node {
     L.perm_in = pin.as<int>();
     L.perm_out = pout.as<int>();
     L.scale = scale;
+    if (list) return launch_conv_list(int(m), rader, L, st);
     return launch_conv_fused(int(m), e, minb, rader, L, st);
   }
   std::string describe() const override {
     std::ostringstream o;
-    o << "(" << (rader ? "rader" : "bluestein") << "-fused n=" << n << " m=" << m << " e=" << e << " minb=" << minb
+    o << "(" << (rader ? "rader" : "bluestein") << "-fused n=" << n << " m=" << m;
+    if (list) {
+      o << " list)";
+      return o.str();
+    }
+    o << " e=" << e << " minb=" << minb
       << " g=" << g << ")";
     return o.str();
   }
@@ -277,6 +284,48 @@ int64_t conv_fused_length(int64_t n) {
   return m <= 8192 ? m : 0;
 }
 
+// what the fused kernels share: stage twiddles and the algorithm's tables
+static bool conv_tables(ConvFusedNode& node, int dir, const std::vector<float2>& tw, std::string* why) {
+  std::vector<cd> b;
+  cudaError_t err = node.tw.upload(tw);
+  if (node.rader) {
+    std::vector<int> pin, pout;
+    rader_tables(node.n, dir, node.m, pin, pout, b);
+    if (err == cudaSuccess) err = node.pin.upload(pin);
+    if (err == cudaSuccess) err = node.pout.upload(pout);
+  } else {
+    const std::vector<cd> w = bluestein_chirp(node.n, dir);
+    b = bluestein_kernel(w, node.m);
+    if (err == cudaSuccess) err = node.chirp.upload(to_f2(w, 1.0));
+  }
+  if (err == cudaSuccess) err = node.spec.upload(to_f2(host_fft(b, -1), 1.0 / double(node.m)));
+  if (err != cudaSuccess && why) *why = "device allocation failed";
+  return err == cudaSuccess;
+}
+
+// The kernel for convolution lengths between the powers of two, when the list
+// has one that is long enough and shorter than the power of two.
+static std::unique_ptr<Node> make_conv_list(int64_t n, const Layout& lay, int dir, float scale, std::string* why) {
+  const bool rader = use_rader(n);
+  const std::vector<int> l = conv_list_radices(rader ? 2 * n - 3 : 2 * n - 1);
+  if (l.empty()) return nullptr;
+  const int64_t m = int64_t(l[0]) * l[1] * l[2], p2 = conv_fused_length(n);
+  if (m > p2) return nullptr;
+  auto node = std::make_unique<ConvFusedNode>();
+  node->rader = rader;
+  node->list = true;
+  node->n = n;
+  node->m = m;
+  node->lay = lay;
+  node->scale = scale;
+  std::vector<float2> tw, inv;
+  make_desc(int(m), {l[0], l[1], l[2]}, tw);
+  make_desc(int(m), {l[1], l[2], l[0]}, inv);
+  tw.insert(tw.end(), inv.begin(), inv.end());
+  if (!conv_tables(*node, dir, tw, why)) return nullptr;
+  return node;
+}
+
 // e = 0: the default shape for the length (PLFFT_B200_CONV_E / _MINB / _G
 // override it), else the given shape
 std::unique_ptr<Node> make_conv_fused(int64_t n, const Layout& lay, int dir, float scale, std::string* why, int e_req,
@@ -284,6 +333,8 @@ std::unique_ptr<Node> make_conv_fused(int64_t n, const Layout& lay, int dir, flo
   if (std::getenv("PLFFT_B200_CONV_UNFUSED")) return nullptr;
   const int64_t m = conv_fused_length(n);
   if (m == 0) return nullptr;
+  if (!e_req && !std::getenv("PLFFT_B200_CONV_E") && !std::getenv("PLFFT_B200_CONV_POW2"))
+    if (auto l = make_conv_list(n, lay, dir, scale, why)) return l;
   const bool rader = use_rader(n);
   const auto shapes = conv_fused_shapes(int(m));
   if (shapes.empty()) return nullptr;
@@ -336,23 +387,7 @@ std::unique_ptr<Node> make_conv_fused(int64_t n, const Layout& lay, int dir, flo
   for (int i = 0; i < ke; ++i) radices.push_back(e);
   std::vector<float2> tw;
   make_desc(int(m), radices, tw);
-  std::vector<cd> b;
-  cudaError_t err = node->tw.upload(tw);
-  if (rader) {
-    std::vector<int> pin, pout;
-    rader_tables(n, dir, m, pin, pout, b);
-    if (err == cudaSuccess) err = node->pin.upload(pin);
-    if (err == cudaSuccess) err = node->pout.upload(pout);
-  } else {
-    const std::vector<cd> w = bluestein_chirp(n, dir);
-    b = bluestein_kernel(w, m);
-    if (err == cudaSuccess) err = node->chirp.upload(to_f2(w, 1.0));
-  }
-  if (err == cudaSuccess) err = node->spec.upload(to_f2(host_fft(b, -1), 1.0 / double(m)));
-  if (err != cudaSuccess) {
-    if (why) *why = "device allocation failed";
-    return nullptr;
-  }
+  if (!conv_tables(*node, dir, tw, why)) return nullptr;
   return node;
 }
 

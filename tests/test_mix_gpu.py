@@ -58,7 +58,7 @@ def test_c2c_fp64(n, strided):
 
 # binary16 buffers on 4-byte and on odd 2-byte boundaries, strided and dense:
 # one rounding of the output (2^-11) on top of FP32
-@pytest.mark.parametrize("n", [2, 16, 100, 1000, 1024, 4096])
+@pytest.mark.parametrize("n", [2, 16, 64, 100, 128, 512, 1000, 1024, 2048, 4096, 8192])
 @pytest.mark.parametrize("offset", [0, 1])
 @pytest.mark.parametrize("strided", [False, True])
 def test_c2c_fp16(n, offset, strided):
@@ -135,3 +135,21 @@ def test_r2c_in_place_dense():
     plan.execute(buf.data_ptr(), buf.data_ptr())
     got = buf.cpu().numpy().view(np.complex64).reshape(hm, h)
     assert oracle.rel_l2(got, np.fft.rfft(x.reshape(hm, n).astype(np.float64))) <= oracle.fp32_tol(n), plan.describe()
+
+
+# Rader and Bluestein convolutions over the listed lengths between the powers
+# of two: the first and last n of each, dense and interleaved, odd batches
+@pytest.mark.parametrize("n", [263, 317, 383, 521, 577, 641, 761, 1031, 1151, 1153, 1279, 1531, 1223])
+@pytest.mark.parametrize("direction", [-1, 1])
+def test_conv_list(n, direction):
+    import torch
+
+    for hm in (1, 7):
+        for s, d in [(1, n + 1), (hm + 1, 1)]:
+            x = seeded_complex(span(hm, d, n, s), n)
+            y = torch.zeros(x.size, dtype=torch.complex64, device="cuda")
+            plan = plfft.make_plan("c2c", n, hm, s, d, s, d, direction=direction)
+            plan.execute(to_dev(x).data_ptr(), y.data_ptr())
+            ref = oracle.c2c(gather(x, hm, d, n, s).astype(np.complex128), direction, method="fft")
+            got = gather(y.cpu().numpy(), hm, d, n, s)
+            assert oracle.rel_l2(got, ref) <= oracle.fp32_tol(n), plan.describe()
