@@ -25,11 +25,12 @@
 namespace plfft_b200 {
 
 // The on-chip transforms run the stages of the mixed-radix engine (mix.cuh)
-// with the stage list of the task in shared memory.  512 threads at 64
-// registers, two CTAs per SM: 32 warps hide the loads of one CTA's tile
-// behind the other's arithmetic, and 72 KB of tile per CTA keep 32 four-step
-// columns of 256 (whole 256-byte segments) together.
-constexpr int kGroupThreads = 512;
+// with the stage list of the task in shared memory.  256 threads at 64
+// registers and 36 KB of tile, four CTAs per SM: while some tiles wait for
+// their loads or at a barrier the others compute (two CTAs of 512 threads
+// took 807 us on the 4000-transform mix, these 727), and 16 four-step columns of 256 are
+// whole 128-byte segments.
+constexpr int kGroupThreads = 256, kGroupPerSm = 4;
 
 __device__ __forceinline__ float2 group_conj(float2 v, bool on) { return on ? make_float2(v.x, -v.y) : v; }
 
@@ -211,28 +212,44 @@ __device__ void run_conv(const GTask& T, const MixDesc& d, const GroupPhase& P, 
   }
 }
 
-__global__ void __launch_bounds__(kGroupThreads, 2) grouped_kernel(const GroupPhase P) {
+__global__ void __launch_bounds__(kGroupThreads, kGroupPerSm) grouped_kernel(const GroupPhase P) {
   extern __shared__ float2 smem[];
-  __shared__ int cur;
-  __shared__ GTask T;
-  __shared__ MixDesc d;
-  for (;;) {
-    if (threadIdx.x == 0) cur = atomicAdd(P.counter, 1);
-    __syncthreads();
-    const int t = cur;
-    if (t >= P.ntasks) break;
-    static_assert(sizeof(GTask) % 4 == 0 && sizeof(MixDesc) % 4 == 0, "copied word by word");
-    const int* tsrc = reinterpret_cast<const int*>(P.tasks + t);
-    const int* dsrc = reinterpret_cast<const int*>(P.descs + P.tasks[t].desc);
-    for (int i = threadIdx.x; i < int(sizeof(GTask) / 4); i += blockDim.x) reinterpret_cast<int*>(&T)[i] = tsrc[i];
-    for (int i = threadIdx.x; i < int(sizeof(MixDesc) / 4); i += blockDim.x) reinterpret_cast<int*>(&d)[i] = dsrc[i];
-    __syncthreads();
+  // tasks in hand: the current one and the next, whose description is on its
+  // way to shared memory while the current one runs, as is the index of the
+  // one after it (fetched one after the other they cost 2 us a task)
+  __shared__ GTask hand[2];
+  __shared__ int index[2];
+  static_assert(sizeof(GTask) % 8 == 0, "copied eight bytes at a time");
+  auto fetch = [&](int slot, int t) {
+    if (t >= P.ntasks) return;
+    const unsigned char* from = reinterpret_cast<const unsigned char*>(P.tasks + t);
+    unsigned char* to = reinterpret_cast<unsigned char*>(&hand[slot]);
+    for (int i = 8 * threadIdx.x; i < int(sizeof(GTask)); i += 8 * blockDim.x) cp_async8(to + i, from + i);
+  };
+  // the first task is the CTA's own, the others come from the counter
+  if (threadIdx.x == 0) {
+    index[0] = blockIdx.x;
+    index[1] = gridDim.x + atomicAdd(P.counter, 1);
+  }
+  __syncthreads();
+  fetch(0, index[0]);
+  cp_async_wait_all();
+  __syncthreads();
+  for (int slot = 0;; slot ^= 1) {
+    if (index[slot] >= P.ntasks) break;
+    fetch(slot ^ 1, index[slot ^ 1]);
+    int after = 0;
+    if (threadIdx.x == 0) after = gridDim.x + atomicAdd(P.counter, 1);
+    __syncthreads();  // index[slot] is read by all before it is replaced below
+    const GTask& T = hand[slot];
     switch (T.type) {
-      case GT_TILE: run_tile(T, d, P, smem); break;
-      case GT_RADER: run_conv<true>(T, d, P, smem); break;
-      case GT_BLUE: run_conv<false>(T, d, P, smem); break;
+      case GT_TILE: run_tile(T, T.d, P, smem); break;
+      case GT_RADER: run_conv<true>(T, T.d, P, smem); break;
+      case GT_BLUE: run_conv<false>(T, T.d, P, smem); break;
       default: break;
     }
+    cp_async_wait_all();
+    if (threadIdx.x == 0) index[slot] = after;
     __syncthreads();
   }
   // the last CTA out resets the counters for the next launch / graph replay
@@ -247,7 +264,7 @@ __global__ void __launch_bounds__(kGroupThreads, 2) grouped_kernel(const GroupPh
 }
 
 int group_threads() { return kGroupThreads; }
-int group_max_smem_elems() { return 72 * 1024 / int(sizeof(float2)); }
+int group_max_smem_elems() { return 36 * 1024 / int(sizeof(float2)); }
 
 cudaError_t launch_grouped(const GroupPhase& P, int grid, int smem_bytes, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);

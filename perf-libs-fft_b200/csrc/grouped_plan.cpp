@@ -34,7 +34,7 @@ namespace plfft_b200 {
 
 namespace {
 
-constexpr int kGroupOnChip = 8192;  // longest on-chip length of the grouped kernel
+constexpr int kGroupOnChip = 4096;  // longest on-chip length of the grouped kernel
 constexpr int kPhases = 4;
 
 struct Tables {
@@ -68,10 +68,12 @@ struct GroupData {
   DevBuf tasks_dev[kPhases];
   std::vector<MixDesc> descs;
   std::vector<std::shared_ptr<DevBuf>> tws;
+  std::map<int64_t, double> cost_of;
+  std::map<int64_t, int64_t> conv_of;
   std::map<int, MixDesc> laid;                   // stages per length (n = 0: none)
   std::map<int, std::shared_ptr<DevBuf>> tw_of;  // twiddles per length
   std::map<std::tuple<int, int, bool, bool>, int> desc_of;
-  DevBuf descs_dev, tws_dev;
+  DevBuf tws_dev;
   std::map<int64_t, std::unique_ptr<Tables>> rader, blue;
   std::map<int64_t, std::unique_ptr<DevBuf>> lo, hi;  // two-level tables per length
   std::map<int64_t, int> lbits;
@@ -220,18 +222,51 @@ struct GroupData {
     return t.get();
   }
 
-  // split m = m1 * m2 for tiles: m1 (column length) small for coalesced
-  // column tiles, both on chip
-  bool split(int64_t m, int64_t& m1, int64_t& m2) {
-    int64_t best = 0;
-    for (int64_t d = 2; d * d <= m; ++d) {
-      if (m % d) continue;
-      if (onchip(d, 1) && onchip(m / d, 1)) best = d;
+  // instructions per element of an on-chip length, more for tiles narrower
+  // than 64 bytes
+  double tile_cost(int64_t L) {
+    auto it = cost_of.find(L);
+    if (it != cost_of.end()) return it->second;
+    double c = -1;
+    if (onchip(L)) {
+      const int width = tile_count(int(L), shape.tile_cap);
+      c = mix_stage_cost(L, std::min(shape.max_radix, 16)) + (width < 8 ? 20.0 * (8.0 / width - 1.0) : 0.0);
     }
-    if (!best) return false;
-    m1 = best;
-    m2 = m / best;
-    return true;
+    return cost_of[L] = c;
+  }
+
+  // split m = m1 * m2 for tiles, both on chip, m1 <= m2: the cheapest pair of
+  // stage lists (few stages first: 210 x 192 beats 200 x 200); -1 if none
+  double split(int64_t m, int64_t& m1, int64_t& m2) {
+    double best = -1;
+    for (int64_t d = 2; d * d <= m; ++d) {
+      if (m % d || !is_smooth(d) || !is_smooth(m / d)) continue;
+      const double a = tile_cost(d), b = tile_cost(m / d);
+      if (a < 0 || b < 0 || (best >= 0 && a + b > best)) continue;
+      best = a + b;
+      m1 = d;
+      m2 = m / d;
+    }
+    return best;
+  }
+
+  // convolution length of a long Bluestein transform: of the smooth lengths
+  // up to a twentieth above 2n - 1, the one whose passes cost least
+  int64_t long_conv_length(int64_t n) {
+    auto it = conv_of.find(n);
+    if (it != conv_of.end()) return it->second;
+    const int64_t need = 2 * n - 1;
+    int64_t best_m = next_smooth(need), m1 = 0, m2 = 0;
+    double best = -1;
+    for (int64_t m = best_m; m <= need + need / 20; m = next_smooth(m + 1)) {
+      const double c = split(m, m1, m2);
+      // 30: the loads, stores and twiddles of two passes
+      if (c >= 0 && (best < 0 || (c + 30.0) * double(m) < best)) {
+        best = (c + 30.0) * double(m);
+        best_m = m;
+      }
+    }
+    return conv_of[n] = best_m;
   }
 
   GTask base_task(int type, int dir_, int n, int cnt, int d) {
@@ -252,8 +287,8 @@ struct GroupData {
   // m cannot be split.
   bool add_four_step(int64_t m, int tdir, int pcol, int prow, int in_buf, int64_t in_off, int out_buf, int64_t out_off,
                      int64_t s1, const GTask& pro, const GTask& epi) {
-    int64_t m1, m2;
-    if (!split(m, m1, m2)) return false;
+    int64_t m1 = 0, m2 = 0;
+    if (split(m, m1, m2) < 0) return false;
     const TwoLevel tl = two_level(m);
     int shift = 0;
     while ((1 << shift) < tl.l) ++shift;
@@ -341,7 +376,7 @@ struct GroupData {
         plans[i] = {onchip(n - 1) ? 1 : 4, n - 1};
       } else {
         const int64_t m = next_smooth(2 * n - 1);
-        plans[i] = {onchip(m) ? 2 : 5, m};
+        plans[i] = onchip(m) ? Plan{2, m} : Plan{5, long_conv_length(n)};
       }
     }
     // one slot per transform for the long ones (sum0 slots at the end)
@@ -460,7 +495,7 @@ struct GroupData {
     // device copies of descriptors, twiddle pointers, tasks (longest first)
     std::vector<const float2*> twp(tws.size());
     for (size_t k = 0; k < tws.size(); ++k) twp[k] = tws[k]->as<float2>();
-    if (descs_dev.upload(descs) != cudaSuccess || tws_dev.upload(twp) != cudaSuccess) return false;
+    if (tws_dev.upload(twp) != cudaSuccess) return false;
     int max_elems = 1;
     for (int p = 0; p < kPhases; ++p) {
       auto cost = [](const GTask& t) {
@@ -469,12 +504,13 @@ struct GroupData {
       };
       std::stable_sort(tasks[p].begin(), tasks[p].end(),
                        [&](const GTask& a, const GTask& b) { return cost(a) > cost(b); });
-      for (const GTask& t : tasks[p]) {
+      for (GTask& t : tasks[p]) {
         if (t.desc < 0) {
           why = "device allocation failed";
           return false;
         }
         const MixDesc& d = descs[t.desc];
+        t.d = d;
         max_elems = std::max(max_elems, d.c * d.ld * (d.inplace ? 1 : 2));
       }
       if (!tasks[p].empty() && tasks_dev[p].upload(tasks[p]) != cudaSuccess) return false;
@@ -497,7 +533,6 @@ struct GroupData {
       GroupPhase P{};
       P.tasks = tasks_dev[p].as<GTask>();
       P.ntasks = int(tasks[p].size());
-      P.descs = descs_dev.as<MixDesc>();
       P.tws = tws_dev.as<const float2*>();
       P.bases[0] = const_cast<float2*>(static_cast<const float2*>(in));
       P.bases[1] = static_cast<float2*>(out);

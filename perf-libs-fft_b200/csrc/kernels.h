@@ -215,11 +215,11 @@ struct GTask {
   TwoLevel tw2;
   int tw2_shift;  // log2 of tw2.l
   float scale;
+  MixDesc d;  // stage 0 has a row of ones in its twiddle table
 };
 struct GroupPhase {
   const GTask* tasks;
   int ntasks;
-  const MixDesc* descs;  // stage 0 has a row of ones in its twiddle table
   const float2* const* tws;
   float2* bases[kGroupBuffers];
   int* counter;

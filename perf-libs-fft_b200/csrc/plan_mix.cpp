@@ -77,6 +77,12 @@ std::vector<int> mix_radices(int64_t n, int max_radix) {
   return best;
 }
 
+double mix_stage_cost(int64_t n, int max_radix) {
+  double c = 0;
+  for (int r : mix_radices(n, max_radix)) c += radix_cost(r);
+  return c;
+}
+
 static bool mix_layout(MixDesc& d, const std::vector<int>& radices, int elem_bytes = 16) {
   const int n = d.n;
   d.nstages = int(radices.size());
@@ -452,7 +458,12 @@ std::unique_ptr<Node> make_mix_real(int kind, int64_t n, const Layout& lay, floa
   const int64_t m = n / 2;
   auto node = std::make_unique<MixRealNode>();
   MixDesc& d = node->base.d;
-  if (!mix_shape(d, m, lay.howmany, false, false, 2, mix_real_last_staged(kind))) return nullptr;
+  int creq = 0;
+  if (const char* v = std::getenv("PLFFT_B200_MIX_C")) creq = std::max(0, std::atoi(v));
+  const bool staged = mix_real_last_staged(kind);
+  if (!mix_shape(d, m, lay.howmany, false, false, 2, staged, creq) &&
+      !(creq && mix_shape(d, m, lay.howmany, false, false, 2, staged)))
+    return nullptr;
   std::vector<float2> tab = mix_twiddle_list<float2>(d);
   const bool iv = kind == FR_DCT4 || kind == FR_DST4;
   const size_t post_off = tab.size();

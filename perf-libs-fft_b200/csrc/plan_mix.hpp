@@ -13,6 +13,8 @@ namespace plfft_b200 {
 // radices 2..16 whose product is n, cheapest stage list first found; empty
 // if n has a prime factor above 13
 std::vector<int> mix_radices(int64_t n, int max_radix);
+// instructions per element of that list's stages
+double mix_stage_cost(int64_t n, int max_radix);
 // radices, tile width, threads and buffers for length n and `count`
 // transforms, `lanes` of them per engine element (FP32 2, FP64 1); c_req > 0
 // asks for a tile width.  False: not on chip.
