@@ -276,10 +276,12 @@ class Plan:
         _check(st, "plfft_plan_execute")
 
     def execute_async(self, inp, out, workspace=0, stream=0):
-        st = lib().plfft_cuda_execute_async(self.handle, ctypes.c_void_p(int(inp)), ctypes.c_void_p(int(out)),
-                                            ctypes.c_void_p(int(workspace)) if workspace else None,
-                                            ctypes.c_void_p(int(stream)) if stream else None)
-        _check(st, "plfft_cuda_execute_async")
+        # ints go to the c_void_p parameters as they are: this call is what a
+        # short transform waits for
+        st = _lib.plfft_cuda_execute_async(self.handle, int(inp), int(out), int(workspace) if workspace else None,
+                                           int(stream) if stream else None)
+        if st:
+            _check(st, "plfft_cuda_execute_async")
 
     def device_status(self, stream=0):
         """plfft_cuda_plan_get_device_status: drains `stream`, returns (and
@@ -339,10 +341,9 @@ class Group:
         self.handle = h
 
     def execute_async(self, d_in, d_out, stream=0):
-        st = lib().plfft_cuda_group_execute_async(self.handle, ctypes.c_void_p(int(d_in)),
-                                                  ctypes.c_void_p(int(d_out)),
-                                                  ctypes.c_void_p(int(stream)) if stream else None)
-        _check(st, "plfft_cuda_group_execute_async")
+        st = _lib.plfft_cuda_group_execute_async(self.handle, int(d_in), int(d_out), int(stream) if stream else None)
+        if st:
+            _check(st, "plfft_cuda_group_execute_async")
 
     def launch_count(self):
         return lib().plfft_cuda_group_get_launch_count(self.handle)
