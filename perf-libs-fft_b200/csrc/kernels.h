@@ -251,7 +251,7 @@ struct RealFusedLaunch {
                             // element 0 (DST-III: element N-1) times 2
 };
 bool real_fused_supported(int64_t m);
-int real_fused_e(int m);
+int real_fused_e(int kind, int m);
 cudaError_t launch_real_fused(int kind, int m, const RealFusedLaunch& L, cudaStream_t st);
 
 // One pass of a power-of-two four-step transform (fourstep.cu): `count`

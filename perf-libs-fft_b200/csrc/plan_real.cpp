@@ -279,10 +279,10 @@ std::unique_ptr<Node> make_real_fused_node(int kind, int64_t n, const Layout& la
   if (!real_fused_supported(n / 2))
     return std::getenv("PLFFT_B200_NO_REAL_HALF") ? nullptr : make_mix_real(kind, n, lay, scale, wmode);
   const int m = int(n / 2);
-  int e = real_fused_e(m);
+  int e = real_fused_e(kind, m);
   if (const char* v = std::getenv("PLFFT_B200_RF_E"))  // launch-shape experiments
-    if (m == 512 && std::atoi(v) == 32) e = 32;
-  if (e_override && (e_override == e || (m == 512 && e_override == 32))) e = e_override;
+    if (m == 512 && (std::atoi(v) == 16 || std::atoi(v) == 32)) e = std::atoi(v);
+  if (e_override && (e_override == e || (m == 512 && (e_override == 16 || e_override == 32)))) e = e_override;
   std::vector<int> radices;
   int rest = m, ke = 0;
   while (rest % e == 0 && rest > 1) {
@@ -315,8 +315,8 @@ std::unique_ptr<Node> make_real_fused_node(int kind, int64_t n, const Layout& la
   node->base.idist = lay.idist;
   node->base.odist = lay.odist;
   // 128 threads, but one transform where it spans several warps: its barriers
-  // then hold up no other (R2C + C2R N=4096 x 8192, 64 threads each: 132 us
-  // with two transforms to a CTA, 127 with one)
+  // then hold up no other (R2C + C2R N=4096 x 8192 at 128 threads each:
+  // 140 us with two transforms to a CTA, 120 with one)
   node->base.g = t > 32 ? 1 : std::max(1, 128 / t);
   if (const char* v = std::getenv("PLFFT_B200_RF_G")) node->base.g = std::max(1, std::atoi(v));
   if (g_override) node->base.g = g_override;

@@ -312,16 +312,22 @@ cudaError_t run_real_fused(const RealFusedLaunch& L, cudaStream_t st) {
   return launch_pdl(real_fused_kernel<M, E, KIND>, dim3(unsigned(blocks)), dim3(T * L.g), size_t(smem), st, L);
 }
 
-// every length of one kind (m = 512 has a 16- and a 32-element form)
+// every length of one kind, at real_fused_e elements per thread (m = 512 also
+// has other forms for the autotuner)
 template <int KIND>
 cudaError_t launch_real_fused_kind(int m, const RealFusedLaunch& L, cudaStream_t st) {
+  constexpr bool III = KIND == FR_DCT3 || KIND == FR_DST3;
+  constexpr bool IV = KIND == FR_DCT4 || KIND == FR_DST4;
   switch (m) {
     case 64: return run_real_fused<64, 16, KIND>(L, st);
     case 128: return run_real_fused<128, 16, KIND>(L, st);
     case 256: return run_real_fused<256, 16, KIND>(L, st);
-    case 512: return L.e == 32 ? run_real_fused<512, 32, KIND>(L, st) : run_real_fused<512, 16, KIND>(L, st);
-    case 1024: return run_real_fused<1024, 32, KIND>(L, st);
-    case 2048: return run_real_fused<2048, 32, KIND>(L, st);
+    case 512:
+      if constexpr (III)
+        if (L.e == 8) return run_real_fused<512, 8, KIND>(L, st);
+      return L.e == 32 ? run_real_fused<512, 32, KIND>(L, st) : run_real_fused<512, 16, KIND>(L, st);
+    case 1024: return run_real_fused<1024, III ? 16 : 32, KIND>(L, st);
+    case 2048: return run_real_fused<2048, IV ? 32 : 16, KIND>(L, st);
     case 4096: return run_real_fused<4096, 16, KIND>(L, st);
     case 8192: return run_real_fused<8192, 32, KIND>(L, st);
   }
