@@ -276,17 +276,21 @@ __host__ __device__ constexpr int fx_pitch(int n) { return ((17 * (n / 16) + 15)
 // whole sectors, and every load of a thread is in flight at once.  Bound by
 // integer issue, so UNIT (both strides 1) folds the addresses into the
 // instructions: Q0.15 N=256 x 16384 (33.5 MB) 15.2 us with the members staged
-// through shared memory first, 11.5 us so.
+// through shared memory first, 11.5 us so, 11.3 with the twiddles fetched
+// before the wait for the previous launch.
 template <int N, int DIR, int B, bool UNIT>
 __global__ void __launch_bounds__(256) fx_two_stage_kernel(const FixedLaunch L) {
   using W = typename Fx<B>::W;
-  griddep_wait();  // launched programmatically (launch_pdl.cuh)
-  griddep_launch_dependents();
   constexpr int M = N / 16, SM = ilog2_c(M);
   constexpr int PITCH = fx_pitch(N);
   extern __shared__ __align__(16) unsigned char fsm[];
   short4* tw = reinterpret_cast<short4*>(fsm);  // (c, s, cvt(-s), c)
   W* tile = reinterpret_cast<W*>(tw + 15 * (M - 1 > 0 ? M - 1 : 1));
+  // the plan's table, which no kernel writes, before the wait for the
+  // previous launch (launch_pdl.cuh)
+  for (int i = threadIdx.x; i < 15 * (M - 1); i += blockDim.x) tw[i] = L.tw[i];
+  griddep_wait();
+  griddep_launch_dependents();
   const int G = blockDim.x / 16;
   const int64_t b0 = int64_t(blockIdx.x) * G;
   const int64_t left = L.howmany - b0;
@@ -300,7 +304,6 @@ __global__ void __launch_bounds__(256) fx_two_stage_kernel(const FixedLaunch L) 
 #pragma unroll
     for (int q = 0; q < M; ++q) w[q] = x[16 * q * is];
   }
-  for (int i = threadIdx.x; i < 15 * (M - 1); i += blockDim.x) tw[i] = L.tw[i];
   if (g < cnt) {  // stage 1: length-M codelet down column c
     qc a[M], r[M];
 #pragma unroll
