@@ -14,7 +14,9 @@
 
 namespace plfft_b200 {
 
-template <int N, int E, int DIR>
+// PAIRS: both buffers 4-byte aligned; else, on an odd multiple of two bytes,
+// scalar accesses
+template <int N, int E, int DIR, bool PAIRS>
 __global__ void __launch_bounds__(pow2_max_threads<E>(), pow2_min_blocks<E>())
     c2c_pow2_half_kernel(const Pow2HalfLaunch L) {
   griddep_wait();  // launched programmatically (launch_pdl.cuh)
@@ -35,8 +37,15 @@ __global__ void __launch_bounds__(pow2_max_threads<E>(), pow2_min_blocks<E>())
   };
   const __half2* src = static_cast<const __half2*>(L.in) + (live ? b * L.idist : 0);
   __half2 h[E];
+  if constexpr (PAIRS) {
 #pragma unroll
-  for (int q = 0; q < E; ++q) h[q] = live ? src[t + T * q] : __half2half2(__ushort_as_half(0));
+    for (int q = 0; q < E; ++q) h[q] = live ? src[t + T * q] : __half2half2(__ushort_as_half(0));
+  } else {
+    const __half* s = reinterpret_cast<const __half*>(src);
+#pragma unroll
+    for (int q = 0; q < E; ++q)
+      h[q] = live ? __halves2half2(s[2 * (t + T * q)], s[2 * (t + T * q) + 1]) : __half2half2(__ushort_as_half(0));
+  }
   float2 v[E];
 #pragma unroll
   for (int q = 0; q < E; ++q) v[q] = __half22float2(h[q]);
@@ -45,7 +54,15 @@ __global__ void __launch_bounds__(pow2_max_threads<E>(), pow2_min_blocks<E>())
   if (!live) return;
   __half2* dst = static_cast<__half2*>(L.out) + b * L.odist;
 #pragma unroll
-  for (int q = 0; q < E; ++q) dst[t + T * q] = __float22half2_rn(cscale(v[q], L.scale));
+  for (int q = 0; q < E; ++q) {
+    const __half2 y = __float22half2_rn(cscale(v[q], L.scale));
+    if constexpr (PAIRS) {
+      dst[t + T * q] = y;
+    } else {
+      reinterpret_cast<__half*>(dst)[2 * (t + T * q)] = __low2half(y);
+      reinterpret_cast<__half*>(dst)[2 * (t + T * q) + 1] = __high2half(y);
+    }
+  }
 }
 
 template <int N, int E>
@@ -53,7 +70,8 @@ static cudaError_t run_half(int dir, Pow2HalfLaunch L, cudaStream_t st) {
   constexpr int T = N / E;
   L.g = T >= 128 ? 1 : 128 / T;
   const int smem = L.g * ((spad_len_c(N) + 1) & ~1) * int(sizeof(float2));
-  auto k = dir < 0 ? c2c_pow2_half_kernel<N, E, -1> : c2c_pow2_half_kernel<N, E, 1>;
+  auto k = L.pairs ? (dir < 0 ? c2c_pow2_half_kernel<N, E, -1, true> : c2c_pow2_half_kernel<N, E, 1, true>)
+                   : (dir < 0 ? c2c_pow2_half_kernel<N, E, -1, false> : c2c_pow2_half_kernel<N, E, 1, false>);
   const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(k), smem);
   if (e != cudaSuccess) return e;
   const int64_t grid = (L.howmany + L.g - 1) / L.g;

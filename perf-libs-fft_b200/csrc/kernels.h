@@ -347,14 +347,14 @@ int fourstep_cluster_smem();
 int fourstep_cluster_capacity();
 cudaError_t launch_fourstep_cluster(int dir, const FourStepClusterLaunch& L, int max_clusters, cudaStream_t st);
 
-// Power-of-two C2C of binary16 (re, im) pairs, 64 <= n <= 8192, unit stride,
-// 4-byte aligned buffers (c2c_pow2_half.cu); the stage list has radix
+// Power-of-two C2C of binary16 (re, im) pairs, 64 <= n <= 8192, unit stride
+// (c2c_pow2_half.cu; pairs: both buffers 4-byte aligned); the stage list has radix
 // pow2_half_e(n) stages after a leftover one
 struct Pow2HalfLaunch {
   const void* in;
   void* out;
   int64_t howmany, idist, odist;
-  int g;
+  int g, pairs;
   float scale;
   const float2* tw;
 };

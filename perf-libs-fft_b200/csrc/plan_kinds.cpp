@@ -201,8 +201,7 @@ static std::unique_ptr<Node> make_half_node(const ConfigData& c, const Layout& l
   // C2C of an on-chip length: binary16 loads and stores in the transform
   // itself (one launch, 8 bytes per element instead of 40)
   if (c.kind == TKind::C2C && member_in_place(c, lay))
-    if (auto t = make_half_c2c(c.n, lay, c.payload, c.scale, [&] { return make_half_chunked(c, lay, why); }, why))
-      return t;
+    if (auto t = make_half_c2c(c.n, lay, c.payload, c.scale, why)) return t;
   return make_half_chunked(c, lay, why);
 }
 

@@ -373,18 +373,14 @@ template std::unique_ptr<Node> make_mix_c2c<double2>(int64_t, const Layout&, int
 
 namespace {
 
-// binary16 power of two: compile-time stages; the tile engine for buffers on
-// an odd multiple of two bytes
+// binary16 power of two: compile-time stages
 struct Pow2HalfNode : Node {
   int n = 0, dir = -1;
   Pow2HalfLaunch base{};
   DevBuf tw;
-  std::unique_ptr<Node> unaligned;
-  size_t workspace() const override { return unaligned->workspace(); }
-  void status_words(std::vector<int*>& out) const override { unaligned->status_words(out); }
-  cudaError_t run(const void* in, void* out, void* ws, cudaStream_t st) const override {
-    if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) % 4) return unaligned->run(in, out, ws, st);
+  cudaError_t run(const void* in, void* out, void*, cudaStream_t st) const override {
     Pow2HalfLaunch L = base;
+    L.pairs = (reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) % 4 == 0;
     L.in = in;
     L.out = out;
     return launch_c2c_pow2_half(n, dir, L, st);
@@ -396,18 +392,14 @@ struct Pow2HalfNode : Node {
 
 }  // namespace
 
-std::unique_ptr<Node> make_half_c2c(int64_t n, const Layout& lay, int dir, double scale,
-                                    const std::function<std::unique_ptr<Node>()>& chunked, std::string* why) {
-  auto mix = make_mix_c2c<float2>(n, lay, dir, scale, true, why);
+std::unique_ptr<Node> make_half_c2c(int64_t n, const Layout& lay, int dir, double scale, std::string* why) {
   // dense powers of two: 7.8 us against 17 us of the tile engine at N=1024 x
   // 4096 (33.5 MB), 6.7 us at N=256 x 16384
-  if (n < 64 || n > 8192 || (n & (n - 1)) || lay.istride != 1 || lay.ostride != 1) return mix;
-  if (!mix) mix = chunked();
-  if (!mix) return nullptr;
+  if (n < 64 || n > 8192 || (n & (n - 1)) || lay.istride != 1 || lay.ostride != 1)
+    return make_mix_c2c<float2>(n, lay, dir, scale, true, why);
   auto node = std::make_unique<Pow2HalfNode>();
   node->n = int(n);
   node->dir = dir;
-  node->unaligned = std::move(mix);
   const int e = pow2_half_e(n);
   std::vector<int> radices;
   int64_t rest = n;

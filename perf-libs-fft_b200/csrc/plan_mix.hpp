@@ -1,6 +1,5 @@
 // Planner interface of the mixed-radix tile engine (plan_mix.cpp).
 #pragma once
-#include <functional>
 #include <memory>
 #include <string>
 #include <vector>
@@ -40,11 +39,8 @@ std::string mix_describe(const MixDesc& d);
 template <class V>
 std::unique_ptr<Node> make_mix_c2c(int64_t n, const Layout& lay, int dir, double scale, bool half, std::string* why);
 
-// one-pass C2C of binary16 buffers; nullptr when n is not an on-chip length.
-// chunked: makes the schedule through FP32 chunks, for unaligned buffers of a
-// length the tile engine does not hold
-std::unique_ptr<Node> make_half_c2c(int64_t n, const Layout& lay, int dir, double scale,
-                                    const std::function<std::unique_ptr<Node>()>& chunked, std::string* why);
+// one-pass C2C of binary16 buffers; nullptr when n is not an on-chip length
+std::unique_ptr<Node> make_half_c2c(int64_t n, const Layout& lay, int dir, double scale, std::string* why);
 // one-pass real transform (FusedRealKind) of even n = 2M with on-chip smooth
 // M, unit strides; nullptr otherwise
 std::unique_ptr<Node> make_mix_real(int kind, int64_t n, const Layout& lay, float scale, int wmode);
