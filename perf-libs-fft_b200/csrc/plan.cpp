@@ -337,6 +337,7 @@ struct C2CFourStepNode : Node {
   int dir = -1;
   DevBuf lo, hi;
   size_t workspace() const override { return size_t(chunk) * size_t(n) * sizeof(float2); }
+  bool reads_batch_first() const override { return chunk >= lay.howmany; }
   int launches() const override { return int(2 * ((lay.howmany + chunk - 1) / chunk)); }
   cudaError_t run(const void* in, void* out, void* ws, cudaStream_t st) const override {
     const float2* x = static_cast<const float2*>(in);
@@ -410,6 +411,7 @@ struct C2CFourStepPow2Node : Node {
   HostWord status;
   void status_words(std::vector<int*>& out) const override { out.push_back(status.p); }
   size_t workspace() const override { return size_t(chunk) * size_t(n) * sizeof(float2); }
+  bool reads_batch_first() const override { return chunk >= lay.howmany; }
   int launches() const override { return int(2 * ((lay.howmany + chunk - 1) / chunk)); }
   bool ring_ok(const void* in, const void* out) const {
     return c1 > 0 && lay.istride == 1 && lay.ostride == 1 && lay.idist % 2 == 0 && lay.odist % 2 == 0 &&
@@ -724,6 +726,7 @@ struct SplitBf16Node : Node {
   FourStepLaunch p1{}, p2{};
   DevBuf tw1, tw2, lo, hi, dftm;
   size_t workspace() const override { return n2 ? size_t(chunk) * size_t(n) * sizeof(float2) : 0; }
+  bool reads_batch_first() const override { return n2 && chunk >= lay.howmany; }
   int launches() const override { return n2 ? int(2 * ((lay.howmany + chunk - 1) / chunk)) : 1; }
   cudaError_t run(const void* in, void* out, void* ws, cudaStream_t st) const override {
     const float2* x = static_cast<const float2*>(in);

@@ -121,6 +121,8 @@ struct Node {
   virtual std::string describe() const = 0;
   // number of kernel launches per run (for launch accounting)
   virtual int launches() const { return 1; }
+  // every input of the batch is read before the first output is written
+  virtual bool reads_batch_first() const { return false; }
   // host-mapped status words its kernels report device-side failures in
   // (bounded waits that ran out); composite nodes add their parts' words
   virtual void status_words(std::vector<int*>& out) const { (void)out; }
@@ -223,6 +225,15 @@ std::vector<std::unique_ptr<Node>> make_real_candidates(int fused_kind, int wrap
 // times make_real_candidates and remembers the winner in wisdom.
 std::unique_ptr<Node> autotune_real(const ConfigData& c, const Layout& lay, int fused_kind, int wrap_kind,
                                     std::string* why, std::string* note);
+
+// An execution that overlaps its input while the outputs do not lie on their
+// own member's inputs must read the whole batch before its first write
+// (plan_kinds.cpp).  `lay` is the layout `node` runs on; adjoint: input and
+// output sides of c swapped.
+std::unique_ptr<Node> guard_in_place(std::unique_ptr<Node> node, const ConfigData& c, const Layout& lay, bool adjoint);
+// Allocates a plan's workspace.  Where there is no room for the copy that a
+// guarded in-place execution needs, the node gives that copy up.
+cudaError_t alloc_workspace(DevBuf& ws, Node& node);
 
 // Adjoint of a plan's transform (same scale, input/output layouts swapped):
 // the conjugate-direction C2C, or the transposed real transform expressed

@@ -122,6 +122,8 @@ struct ConvNode : Node {
   size_t workspace() const override {
     return work_bytes() + sum_bytes() + std::max(fwd->workspace(), bwd->workspace());
   }
+  // (Rader's last launch reads element 0 of each member again)
+  bool reads_batch_first() const override { return !rader && chunk >= lay.howmany; }
   int launches() const override {
     const int64_t chunks = (lay.howmany + chunk - 1) / chunk;
     return int(chunks * (3 + fwd->launches() + bwd->launches()));

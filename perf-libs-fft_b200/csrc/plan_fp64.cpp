@@ -39,6 +39,7 @@ struct F64C2CNode : Node {
   MixLaunch<double2> p1{}, p2{};
   DevBuf tw1, tw2, lo, hi;
   size_t workspace() const override { return n2 ? size_t(chunk * n) * sizeof(double2) : 0; }
+  bool reads_batch_first() const override { return n2 && chunk >= lay.howmany; }
   int launches() const override { return n2 ? int(2 * ((lay.howmany + chunk - 1) / chunk)) : 1; }
   cudaError_t run(const void* in, void* out, void* ws, cudaStream_t st) const override {
     const auto* x = static_cast<const double2*>(in);
@@ -81,6 +82,7 @@ struct F64RealNode : Node {
   int64_t howmany = 1, chunk = 1;
   size_t work_bytes() const { return size_t(chunk * base.n) * sizeof(double2); }
   size_t workspace() const override { return (work_bytes() + 255) / 256 * 256 + c2c->workspace(); }
+  bool reads_batch_first() const override { return chunk >= howmany; }
   int launches() const override { return int((howmany + chunk - 1) / chunk) * (2 + c2c->launches()); }
   cudaError_t run(const void* in, void* out, void* ws, cudaStream_t st) const override {
     F64RealLaunch L = base;

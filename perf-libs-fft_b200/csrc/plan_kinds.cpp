@@ -48,14 +48,68 @@ static int r2r_wrap_kind(int payload) {
 
 // May the members of an aliased batch be transformed one CTA at a time, each
 // member's output written as soon as its own tile is read?  Yes when the
-// outputs of a member lie where its inputs do; other in-place layouts keep
-// the schedules that read the whole batch before the first write.
-static bool member_in_place(const ConfigData& c, const Layout& lay) {
+// outputs of a member lie where its inputs do; other in-place layouts need
+// the whole batch read before the first write.
+static bool member_in_place(const ConfigData& c, const Layout& lay, bool adjoint = false) {
   if (c.alias != PLFFT_IO_MAY_ALIAS || lay.howmany == 1) return true;
   int64_t nin = 0, nout = 0;
   bool ic = false, oc = false;
   io_counts(c, nin, nout, ic, oc);
+  if (adjoint) std::swap(ic, oc);
   return lay.istride == lay.ostride && lay.idist * (ic ? 2 : 1) == lay.odist * (oc ? 2 : 1);
+}
+
+namespace {
+
+// A schedule that writes members while others are still to be read.  Where
+// the buffers of an execution overlap it runs from a copy of its input,
+// which costs one more read and write of that; elsewhere it runs as it is.
+struct InPlaceNode : Node {
+  std::unique_ptr<Node> inner;
+  size_t in_bytes = 0, out_bytes = 0;  // spans of one execution
+  bool copies = true;                  // false: there was no room for the copy
+  size_t inner_ws() const { return (inner->workspace() + 255) & ~size_t(255); }
+  size_t workspace() const override { return copies ? inner_ws() + in_bytes : inner->workspace(); }
+  int launches() const override { return inner->launches(); }
+  bool reads_batch_first() const override { return true; }
+  void status_words(std::vector<int*>& out) const override { inner->status_words(out); }
+  cudaError_t run(const void* in, void* out, void* ws, cudaStream_t st) const override {
+    const uintptr_t i0 = reinterpret_cast<uintptr_t>(in), o0 = reinterpret_cast<uintptr_t>(out);
+    if (i0 >= o0 + out_bytes || o0 >= i0 + in_bytes) return inner->run(in, out, ws, st);
+    if (!copies) return cudaErrorMemoryAllocation;
+    void* copy = static_cast<unsigned char*>(ws) + inner_ws();
+    const cudaError_t e = cudaMemcpyAsync(copy, in, in_bytes, cudaMemcpyDeviceToDevice, st);
+    return e == cudaSuccess ? inner->run(copy, out, ws, st) : e;
+  }
+  std::string describe() const override { return inner->describe() + " (in place: from a copy of the input)"; }
+};
+
+}  // namespace
+
+std::unique_ptr<Node> guard_in_place(std::unique_ptr<Node> node, const ConfigData& c, const Layout& lay, bool adjoint) {
+  if (!node || member_in_place(c, lay, adjoint) || node->reads_batch_first()) return node;
+  int64_t nin = 0, nout = 0;
+  bool ic = false, oc = false;
+  io_counts(c, nin, nout, ic, oc);
+  if (adjoint) {
+    std::swap(nin, nout);
+    std::swap(ic, oc);
+  }
+  const int sb = scalar_bytes(c.data_type);
+  auto g = std::make_unique<InPlaceNode>();
+  g->inner = std::move(node);
+  g->in_bytes = size_t(span(lay.howmany, lay.idist, nin, lay.istride)) * sb * (ic ? 2 : 1);
+  g->out_bytes = size_t(span(lay.howmany, lay.odist, nout, lay.ostride)) * sb * (oc ? 2 : 1);
+  return g;
+}
+
+cudaError_t alloc_workspace(DevBuf& ws, Node& node) {
+  cudaError_t e = ws.alloc(node.workspace());
+  auto* g = dynamic_cast<InPlaceNode*>(&node);
+  if (e == cudaSuccess || !g) return e;
+  cudaGetLastError();
+  g->copies = false;
+  return ws.alloc(node.workspace());
 }
 
 // fused kind of an R2R payload, or -1
@@ -82,9 +136,7 @@ static std::unique_ptr<Node> make_root(const ConfigData& c, const Layout& lay, b
       case TKind::C2R:
       case TKind::R2R: {
         const int wrap = c.kind == TKind::R2C ? RW_R2C : (c.kind == TKind::C2R ? RW_C2R : r2r_wrap_kind(c.payload));
-        int fused = c.kind == TKind::R2C ? FR_R2C : (c.kind == TKind::C2R ? FR_C2R : r2r_fused_kind(c.payload));
-        // the power-of-two kernel's lengths have always run member by member
-        if (!(c.n % 2 == 0 && real_fused_supported(c.n / 2)) && !member_in_place(c, lay)) fused = -1;
+        const int fused = c.kind == TKind::R2C ? FR_R2C : (c.kind == TKind::C2R ? FR_C2R : r2r_fused_kind(c.payload));
         if (tune && c.rigor != PLFFT_ESTIMATE) {
           root = autotune_real(c, lay, fused, wrap, why, note);
           break;
@@ -127,6 +179,9 @@ static std::unique_ptr<Node> make_root(const ConfigData& c, const Layout& lay, b
   } else {
     if (why) *why = "data type not supported on the device path";
   }
+  // (binary16 and fixed-point schedules are chosen by layout where it matters)
+  if (c.data_type == PLFFT_DATA_TYPE_FP32 || c.data_type == PLFFT_DATA_TYPE_FP64)
+    root = guard_in_place(std::move(root), c, lay, false);
   return root;
 }
 
@@ -226,7 +281,7 @@ plfft_status_t build_plan(PlanData& p, std::string* why) {
                 (c.ostride == 1 && c.odist == nout) ||
                 (c.odist == 1 && c.ostride == c.howmany);
 
-  if (p.ws.alloc(p.root->workspace()) != cudaSuccess) {
+  if (alloc_workspace(p.ws, *p.root) != cudaSuccess) {
     if (why) *why = "workspace allocation failed";
     return PLFFT_PLAN_CREATION_FAILED;
   }
@@ -273,8 +328,10 @@ static void build_pipe(const PlanData& p) {
   const int64_t per = (c.howmany + k - 1) / k;
   const int64_t tail = c.howmany - (c.howmany - 1) / per * per;
   std::string why, note;
-  p.pipe_node = make_root(c, Layout{per, c.istride, c.idist, c.ostride, c.odist}, false, &why, &note);
-  if (tail != per) p.pipe_tail = make_root(c, Layout{tail, c.istride, c.idist, c.ostride, c.odist}, false, &why, &note);
+  ConfigData cs = c;  // its two staging buffers never overlap
+  cs.alias = PLFFT_IO_NO_ALIAS;
+  p.pipe_node = make_root(cs, Layout{per, c.istride, c.idist, c.ostride, c.odist}, false, &why, &note);
+  if (tail != per) p.pipe_tail = make_root(cs, Layout{tail, c.istride, c.idist, c.ostride, c.odist}, false, &why, &note);
   if (!p.pipe_node || (tail != per && !p.pipe_tail)) return;
   size_t ws = p.pipe_node->workspace();
   if (p.pipe_tail) ws = std::max(ws, p.pipe_tail->workspace());

@@ -27,6 +27,7 @@ struct RealWrapNode : Node {
     const size_t work = size_t(chunk) * size_t(len) * cbytes();
     return ((work + 255) & ~size_t(255)) + inner_ws();
   }
+  bool reads_batch_first() const override { return chunk >= lay.howmany; }
   int launches() const override {
     const int64_t chunks = (lay.howmany + chunk - 1) / chunk;
     return int(chunks * (2 + inner->launches()));
@@ -112,6 +113,7 @@ struct RealHalfNode : Node {
     if (inner_last) iw = std::max(iw, inner_last->workspace());
     return std::max(work_bytes() + iw, generic->workspace());
   }
+  bool reads_batch_first() const override { return chunk >= lay.howmany && generic->reads_batch_first(); }
   int launches() const override {
     const int64_t chunks = (lay.howmany + chunk - 1) / chunk;
     return int(chunks * (1 + inner->launches()));

@@ -137,6 +137,72 @@ def test_r2c_in_place_dense():
     assert oracle.rel_l2(got, np.fft.rfft(x.reshape(hm, n).astype(np.float64))) <= oracle.fp32_tol(n), plan.describe()
 
 
+# In place with outputs away from their own member's inputs: batches of several
+# CTAs (and of the two or more members that shared one), whose members a CTA
+# may write while another has yet to read them.  Kind, length, members, input
+# and output (stride, distance).
+MOVED = [("c2c", 360, 16, (1, 360), (16, 1)), ("c2c", 360, 700, (1, 360), (700, 1)),
+         ("c2c", 1000, 600, (600, 1), (1, 1001)), ("c2c", 1024, 300, (1, 1024), (300, 1)),
+         ("c2c", 1031, 200, (1, 1031), (200, 1)), ("c2c", 12000, 5, (1, 12000), (5, 1)),
+         ("r2c", 1000, 1500, (1, 1000), (1, 501)), ("c2r", 1000, 1500, (1, 501), (1, 1000)),
+         ("r2c", 4096, 2, (1, 4096), (1, 2049)), ("c2r", 4096, 300, (1, 2049), (1, 4096)),
+         ("dct2", 1000, 900, (1, 1000), (1, 1001)), ("dct2", 1024, 900, (1, 1024), (1, 1025))]
+MOVED64 = [("c2c", 1000, 300, (1, 1000), (300, 1)), ("c2c", 5000, 40, (1, 5000), (40, 1)),
+           ("c2c", 8192, 40, (40, 1), (1, 8192)), ("r2c", 1000, 300, (1, 1000), (1, 501))]
+
+
+def _moved(kind, n, hm, i, o, dtype, adjoint):
+    """one execution in a buffer of its own and one in place, as the output spans' members"""
+    import torch
+
+    h = n // 2 + 1
+    nin, ci = (h, 2) if kind == "c2r" else (n, 2 if kind == "c2c" else 1)
+    nout, co = (h, 2) if kind == "r2c" else (n, 2 if kind == "c2c" else 1)
+    args = (hm, i[0], i[1], o[0], o[1])
+    kw = dict(data_type=plfft.DataType.FP32 if dtype == torch.float32 else plfft.DataType.FP64)
+    if kind == "dct2":
+        kw["r2r_kind"] = plfft.R2RKind.DCT_2
+    plans = [plfft.make_plan("r2r" if kind == "dct2" else kind, n, *args, alias=a, **kw)
+             for a in (plfft.IoAlias.NO_ALIAS, plfft.IoAlias.MAY_ALIAS)]
+    if adjoint:
+        (nin, ci, i), (nout, co, o) = (nout, co, o), (nin, ci, i)
+    si, so = ci * span(hm, i[1], nin, i[0]), co * span(hm, o[1], nout, o[0])
+    x = torch.rand(si, generator=torch.Generator().manual_seed(n), dtype=dtype).cuda()
+    run = [(p.execute_adjoint if adjoint else p.execute) for p in plans]
+    y = torch.zeros(so, dtype=dtype, device="cuda")
+    run[0](x.data_ptr(), y.data_ptr())
+    buf = torch.zeros(max(si, so), dtype=dtype, device="cuda")
+    buf[:si] = x
+    run[1](buf.data_ptr(), buf.data_ptr())
+    apart = torch.zeros(so, dtype=dtype, device="cuda")  # the same plan on two buffers
+    run[1](x.data_ptr(), apart.data_ptr())
+    torch.cuda.synchronize()
+    ctype = {1: None, 2: np.complex64 if dtype == torch.float32 else np.complex128}[co]
+    pick = lambda t: gather(t.cpu().numpy()[:so].view(ctype) if ctype else t.cpu().numpy()[:so], hm, o[1], nout, o[0])
+    return pick(y), pick(buf), pick(apart), plans[1]
+
+
+# the same schedule on the same numbers: equal up to how a CTA's members are
+# grouped, one FP32 (FP64) rounding chain
+@pytest.mark.parametrize("kind,n,hm,i,o", MOVED)
+def test_in_place_moved_members(kind, n, hm, i, o):
+    import torch
+
+    ref, got, apart, plan = _moved(kind, n, hm, i, o, torch.float32, False)
+    assert oracle.rel_l2(got, ref) <= oracle.fp32_tol(n), plan.describe()
+    assert oracle.rel_l2(apart, ref) <= oracle.fp32_tol(n), plan.describe()
+
+
+@pytest.mark.parametrize("kind,n,hm,i,o", MOVED64)
+def test_in_place_moved_members_fp64(kind, n, hm, i, o):
+    import torch
+
+    ref, got, apart, plan = _moved(kind, n, hm, i, o, torch.float64, False)
+    tol = 8 * np.log2(n) * 2.0**-53
+    assert oracle.rel_l2(got, ref) <= tol, plan.describe()
+    assert oracle.rel_l2(apart, ref) <= tol, plan.describe()
+
+
 # Rader and Bluestein convolutions over the listed lengths between the powers
 # of two: the first and last n of each, dense and interleaved, odd batches
 @pytest.mark.parametrize("n", [263, 317, 383, 521, 577, 641, 761, 1031, 1151, 1153, 1279, 1531, 1223])
