@@ -254,7 +254,7 @@ static bool ensure_adjoint(const PlanData& p) {
   std::string why;
   auto node = make_adjoint_node(p.cfg, &why);
   if (!node) return false;
-  if (p.adj_ws.alloc(node->workspace()) != cudaSuccess) return false;
+  if (alloc_workspace(p.adj_ws, *node) != cudaSuccess) return false;
   p.adjoint = std::move(node);
   return true;
 }

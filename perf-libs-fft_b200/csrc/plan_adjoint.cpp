@@ -19,9 +19,7 @@
 
 namespace plfft_b200 {
 
-std::unique_ptr<Node> make_adjoint_node(const ConfigData& c, std::string* why) {
-  // the adjoint reads the plan's output layout and writes its input layout
-  const Layout lay{c.howmany, c.ostride, c.howmany > 1 ? c.odist : 0, c.istride, c.howmany > 1 ? c.idist : 0};
+static std::unique_ptr<Node> make_schedule(const ConfigData& c, const Layout& lay, std::string* why) {
   const float scale = float(c.scale);
   if (c.data_type != PLFFT_DATA_TYPE_FP32) {
     if (why) *why = "adjoint available for FP32 plans";
@@ -64,6 +62,12 @@ std::unique_ptr<Node> make_adjoint_node(const ConfigData& c, std::string* why) {
   }
   if (why) *why = "no adjoint for this transform";
   return nullptr;
+}
+
+std::unique_ptr<Node> make_adjoint_node(const ConfigData& c, std::string* why) {
+  // the adjoint reads the plan's output layout and writes its input layout
+  const Layout lay{c.howmany, c.ostride, c.howmany > 1 ? c.odist : 0, c.istride, c.howmany > 1 ? c.idist : 0};
+  return guard_in_place(make_schedule(c, lay, why), c, lay, true);
 }
 
 }  // namespace plfft_b200

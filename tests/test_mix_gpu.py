@@ -203,6 +203,16 @@ def test_in_place_moved_members_fp64(kind, n, hm, i, o):
     assert oracle.rel_l2(apart, ref) <= tol, plan.describe()
 
 
+# the adjoint of such a plan, in place
+@pytest.mark.parametrize("kind,n,hm,i,o", MOVED)
+def test_adjoint_in_place_moved_members(kind, n, hm, i, o):
+    import torch
+
+    ref, got, apart, plan = _moved(kind, n, hm, i, o, torch.float32, True)
+    assert oracle.rel_l2(got, ref) <= oracle.fp32_tol(n), plan.describe()
+    assert oracle.rel_l2(apart, ref) <= oracle.fp32_tol(n), plan.describe()
+
+
 # Rader and Bluestein convolutions over the listed lengths between the powers
 # of two: the first and last n of each, dense and interleaved, odd batches
 @pytest.mark.parametrize("n", [263, 317, 383, 521, 577, 641, 761, 1031, 1151, 1153, 1279, 1531, 1223])
