@@ -93,9 +93,12 @@ plfft_cuda_plan_get_adjoint_workspace_size(const plfft_plan_t *plan,
  * Transform i has lengths[i] contiguous complex elements starting at element
  * in_offsets[i] of the input buffer and out_offsets[i] of the output buffer
  * (the output regions must not overlap each other or any input region).
- * Every length is accepted: on-chip lengths, Rader primes, Bluestein lengths
- * and four-step lengths all run inside the same persistent kernel, at most
- * four launches (one per dependency phase) replayed as one CUDA graph. */
+ * Every length up to 2^23 is accepted, and longer ones whose four-step or
+ * convolution length is a product of two {2,3,5,7,11,13}-smooth factors of at
+ * most 8192 each: on-chip lengths, Rader primes, Bluestein lengths and
+ * four-step lengths all run inside the same persistent kernel, at most four
+ * launches (one per dependency phase) replayed as one CUDA graph.  Other
+ * lengths fail with PLFFT_PLAN_CREATION_FAILED. */
 typedef struct plfft_cuda_group_t plfft_cuda_group_t;
 plfft_status_t plfft_cuda_group_create(plfft_cuda_group_t **group,
                                        int64_t count, const int64_t *lengths,

@@ -265,9 +265,11 @@ __global__ void __launch_bounds__(kGroupThreads, kGroupPerSm) grouped_kernel(con
 
 int group_threads() { return kGroupThreads; }
 int group_max_smem_elems() { return 36 * 1024 / int(sizeof(float2)); }
+// one CTA per SM, less the task descriptions
+int group_most_smem_elems() { return 220 * 1024 / int(sizeof(float2)); }
 
 cudaError_t launch_grouped(const GroupPhase& P, int grid, int smem_bytes, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+  const cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_kernel), smem_bytes);
   if (e != cudaSuccess) return e;
   grouped_kernel<<<grid, kGroupThreads, smem_bytes, st>>>(P);
   return cudaGetLastError();
@@ -275,8 +277,8 @@ cudaError_t launch_grouped(const GroupPhase& P, int grid, int smem_bytes, cudaSt
 
 int grouped_blocks_per_sm(int smem_bytes) {
   int per = 0;
-  cudaFuncSetAttribute(grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, grouped_kernel, kGroupThreads, smem_bytes);
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(grouped_kernel), smem_bytes) == cudaSuccess)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, grouped_kernel, kGroupThreads, smem_bytes);
   return per < 1 ? 1 : per;
 }
 

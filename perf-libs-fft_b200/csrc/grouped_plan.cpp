@@ -35,6 +35,7 @@ namespace plfft_b200 {
 namespace {
 
 constexpr int kGroupOnChip = 4096;  // longest on-chip length of the grouped kernel
+constexpr int kGroupFactor = 8192;  // longest factor of a four-step length
 constexpr int kPhases = 4;
 
 struct Tables {
@@ -80,7 +81,7 @@ struct GroupData {
   DevBuf counters;
   DevBuf ws;
   size_t ws_bytes = 0;
-  int smem_bytes = 0;
+  int smem_bytes[kPhases] = {};
   int grid[kPhases] = {0, 0, 0, 0};
   int nlarge = 0, nonchip = 0, nrader = 0, nblue = 0, nconv_large = 0;
   bool use_graph = true;
@@ -93,8 +94,9 @@ struct GroupData {
     if (graph) cudaGraphExecDestroy(graph);
   }
 
-  // the tile of cnt transforms of length L, if it fits the kernel's CTA
-  bool tile_fits(int L, int cnt, MixDesc* d = nullptr) {
+  // the tile of cnt transforms of length L, if it fits max_elems elements of
+  // the kernel's shared memory
+  bool tile_fits(int L, int cnt, MixDesc* d = nullptr, int max_elems = group_max_smem_elems()) {
     auto it = laid.find(L);
     if (it == laid.end()) {
       MixDesc t;
@@ -103,7 +105,7 @@ struct GroupData {
     }
     if (it->second.n == 0) return false;
     MixDesc t = it->second;
-    if (!mix_tile_set(t, cnt, group_threads(), group_max_smem_elems())) return false;
+    if (!mix_tile_set(t, cnt, group_threads(), max_elems)) return false;
     if (d) *d = t;
     return true;
   }
@@ -115,7 +117,7 @@ struct GroupData {
     auto it = desc_of.find(key);
     if (it != desc_of.end()) return it->second;
     MixDesc d;
-    if (!tile_fits(L, cnt, &d)) return -1;
+    if (!tile_fits(L, cnt, &d) && !(cnt == 1 && tile_fits(L, 1, &d, group_most_smem_elems()))) return -1;
     d.cf_in = cf_in;
     d.cf_out = cf_out;
     d.cf_mid = cnt >= 16;
@@ -235,9 +237,41 @@ struct GroupData {
     return cost_of[L] = c;
   }
 
+  // shared-memory elements of one transform of length L, any tile size; 0 if
+  // no CTA holds it
+  int single_elems(int64_t L) {
+    MixDesc d;
+    if (L > kGroupFactor || !is_smooth(L) || !tile_fits(int(L), 1, &d, group_most_smem_elems())) return 0;
+    return d.ld * (d.inplace ? 1 : 2);
+  }
+
   // split m = m1 * m2 for tiles, both on chip, m1 <= m2: the cheapest pair of
   // stage lists (few stages first: 210 x 192 beats 200 x 200); -1 if none
   double split(int64_t m, int64_t& m1, int64_t& m2) {
+    const double c = split_small(m, m1, m2);
+    return c >= 0 ? c : split_large(m, m1, m2);
+  }
+
+  // Lengths whose every split has a factor beyond the usual tile (3557763 =
+  // 1089 x 3267, 2^25): tiles of one transform in as much shared memory as
+  // they take, the pair that takes least, so that most CTAs fit an SM.
+  double split_large(int64_t m, int64_t& m1, int64_t& m2) {
+    int best = 0;
+    for (int64_t d = 2; d * d <= m; ++d) {
+      if (m % d || m / d > kGroupFactor) continue;
+      const int a = single_elems(d), b = single_elems(m / d);
+      if (!a || !b || (best && std::max(a, b) >= best)) continue;
+      best = std::max(a, b);
+      m1 = d;
+      m2 = m / d;
+    }
+    if (!best) return -1;
+    const int radix = std::min(shape.max_radix, 16);
+    // 140: a tile one element wide (tile_cost)
+    return mix_stage_cost(m1, radix) + mix_stage_cost(m2, radix) + 2 * 140.0;
+  }
+
+  double split_small(int64_t m, int64_t& m1, int64_t& m2) {
     double best = -1;
     for (int64_t d = 2; d * d <= m; ++d) {
       if (m % d || !is_smooth(d) || !is_smooth(m / d)) continue;
@@ -496,8 +530,8 @@ struct GroupData {
     std::vector<const float2*> twp(tws.size());
     for (size_t k = 0; k < tws.size(); ++k) twp[k] = tws[k]->as<float2>();
     if (tws_dev.upload(twp) != cudaSuccess) return false;
-    int max_elems = 1;
     for (int p = 0; p < kPhases; ++p) {
+      int max_elems = 1;
       auto cost = [](const GTask& t) {
         double c = double(t.cnt) * t.n * std::log2(double(t.n) + 1.0);
         return t.type == GT_TILE ? c : 2.0 * c;
@@ -514,16 +548,15 @@ struct GroupData {
         max_elems = std::max(max_elems, d.c * d.ld * (d.inplace ? 1 : 2));
       }
       if (!tasks[p].empty() && tasks_dev[p].upload(tasks[p]) != cudaSuccess) return false;
+      smem_bytes[p] = max_elems * int(sizeof(float2));
     }
-    smem_bytes = max_elems * int(sizeof(float2));
     if (counters.alloc(2 * kPhases * sizeof(int)) != cudaSuccess ||
         cudaMemset(counters.p, 0, 2 * kPhases * sizeof(int)) != cudaSuccess)
       return false;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int per = grouped_blocks_per_sm(smem_bytes);
     for (int p = 0; p < kPhases; ++p)
-      grid[p] = int(std::min<int64_t>(int64_t(tasks[p].size()), int64_t(per) * sms));
+      grid[p] = int(std::min<int64_t>(int64_t(tasks[p].size()), int64_t(grouped_blocks_per_sm(smem_bytes[p])) * sms));
     return true;
   }
 
@@ -539,7 +572,7 @@ struct GroupData {
       P.bases[2] = ws.as<float2>();
       P.counter = counters.as<int>() + 2 * p;
       P.done = counters.as<int>() + 2 * p + 1;
-      const cudaError_t e = launch_grouped(P, grid[p], smem_bytes, st);
+      const cudaError_t e = launch_grouped(P, grid[p], smem_bytes[p], st);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -583,7 +616,7 @@ struct GroupData {
     o << "(group count=" << count << " " << shape.str() << " onchip=" << nonchip << " rader=" << nrader << " bluestein=" << nblue
       << " four-step=" << nlarge << " long-conv=" << nconv_large << " phases=" << launches() << " tasks=["
       << tasks[0].size() << "," << tasks[1].size() << "," << tasks[2].size() << "," << tasks[3].size()
-      << "] smem=" << smem_bytes << " graph=" << (use_graph ? 1 : 0) << ")";
+      << "] smem=" << *std::max_element(smem_bytes, smem_bytes + kPhases) << " graph=" << (use_graph ? 1 : 0) << ")";
     return o.str();
   }
 };
@@ -597,6 +630,18 @@ struct plfft_cuda_group_t {
 };
 
 extern "C" {
+
+// For the host-side test of the tile rules, not part of the API: how a group
+// splits each four-step (or convolution) length, 1 into usual tiles, 2 into
+// larger ones, 0 not at all.
+void plfft_b200_group_splits(const int64_t* m, int64_t count, unsigned char* how) {
+  GroupData g;
+  for (int64_t i = 0; i < count; ++i) {
+    int64_t m1 = 0, m2 = 0;
+    how[i] = g.split_small(m[i], m1, m2) >= 0 ? 1 : (g.split_large(m[i], m1, m2) >= 0 ? 2 : 0);
+    if (how[i] && m1 * m2 != m[i]) how[i] = 0;
+  }
+}
 
 plfft_status_t plfft_cuda_group_create(plfft_cuda_group_t** group, int64_t count, const int64_t* lengths,
                                        const int64_t* in_offsets, const int64_t* out_offsets,

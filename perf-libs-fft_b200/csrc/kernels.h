@@ -227,7 +227,8 @@ struct GroupPhase {
 };
 cudaError_t launch_grouped(const GroupPhase& P, int grid, int smem_bytes, cudaStream_t st);
 int grouped_blocks_per_sm(int smem_bytes);
-int group_max_smem_elems();
+int group_max_smem_elems();   // of the usual tile
+int group_most_smem_elems();  // of any tile
 int group_threads();
 
 // Fused single-kernel real transforms for N = 2M, M a power of two

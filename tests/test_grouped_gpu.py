@@ -115,3 +115,15 @@ def test_group_tuned_and_wisdom():
     _check([lengths[i] for i in pick], x2, y2, [offs2[i] for i in pick], 1)
     with pytest.raises(plfft.PlfftError):
         _run_group([16, 32], -1, seed=8, rigor=7)
+
+
+# four-step lengths (5314411: the convolution of a Rader prime) none of whose
+# splits fits the usual tile
+@pytest.mark.parametrize("lengths", [[3557763, 100, 1031], [5314411, 64], [1 << 25]])
+@pytest.mark.parametrize("direction", [-1, 1])
+def test_group_large_factors(lengths, direction):
+    g, x, y, offs = _run_group(lengths, direction, seed=9, gap=1)
+    for n, o in zip(lengths, offs):
+        xl = x[o:o + n].astype(np.complex128)
+        ref = np.fft.fft(xl) if direction < 0 else np.fft.ifft(xl) * n
+        assert oracle.rel_l2(y[o:o + n], ref) <= oracle.fp32_tol(n), (n, g.describe())
