@@ -330,10 +330,13 @@ __global__ void __launch_bounds__(MixTraits<V>::threads, 1)
   __syncthreads();
   const int ns = d.nstages;
   if (ns == 1) {
+    // one stage: stored from shared memory, lanes along the dense direction
+    // (C2C n=8 x 524288: 23.5 us, 37.3 with lanes along the transforms)
     const int total = d.c * d.n;
     for (int f = threadIdx.x; f < total; f += blockDim.x) {
-      const int k = f / d.c, c = f - k * d.c;
-      if (c < cnt) io.store1(c, k, buf0[c * d.ld + k]);
+      const int a = d.cf_out ? d.c : d.n, hi = f / a, lo = f - hi * a;
+      const int k = d.cf_out ? hi : lo, c = d.cf_out ? lo : hi;
+      if (c < cnt) io.store1(c, k, mix_ld(buf0 + c * d.ld + k));
     }
     return;
   }

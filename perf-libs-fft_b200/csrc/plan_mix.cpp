@@ -198,8 +198,14 @@ bool mix_shape(MixDesc& d, int64_t n, int64_t count, bool cf_in, bool cf_out, in
   const int max_thr = lanes == 2 ? kMixThreadsPair : kMixThreads64;
   const int held = lanes == 2 ? kMixHeldPair : kMixHeldSingle;
   if (n < 2 || n > 16384) return false;
-  const std::vector<int> radices = mix_radices(n, 16);
+  std::vector<int> radices = mix_radices(n, 16);
   if (radices.empty()) return false;
+  // A single stage gives a whole transform to one thread, and at 14 points and
+  // more a dense side pays for lanes that lie n elements apart: two stages
+  // (us, 2^22 numbers, one / two: C2C n=14 22.6 / 19.8, 15 23.3 / 15.7, 16
+  // 28.2 / 16.8; C2R n=32 47.0 / 13.0; n=12 19.3 / 16.1, but its real kinds
+  // of 1000 members 4.3 / 5.6).
+  if (n >= 14 && radices.size() == 1 && !(cf_in && cf_out)) radices = mix_radices(n, int(n) - 1);
   MixDesc best{};
   double best_cost = -1;
   // strided batches move segments of c consecutive elements: whole 32-byte

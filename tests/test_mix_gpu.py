@@ -34,6 +34,28 @@ def test_c2c_fp32(n, direction):
         assert np.all(got[~touched] == 7.0), "wrote outside the members"
 
 
+# lengths of one radix: stored from shared memory, or from 14 points on a dense
+# batch as two stages
+@pytest.mark.parametrize("n,radices", [(5, "5"), (8, "8"), (12, "12"), (13, "13"), (14, "7x2"), (15, "5x3"), (16, "4x4")])
+def test_c2c_short(n, radices):
+    import torch
+
+    hm = 1001
+    for (s, d), want in [((1, n), radices), ((1, n + 1), radices), ((hm + 1, 1), str(n))]:
+        for dt, ct in [(plfft.DataType.FP32, np.complex64), (plfft.DataType.FP64, np.complex128)]:
+            x = seeded_complex(span(hm, d, n, s), n).astype(ct)
+            y = torch.full((x.size,), 7.0, dtype=to_dev(x).dtype, device="cuda")
+            plan = plfft.make_plan("c2c", n, hm, s, d, s, d, data_type=dt)
+            assert "radices=%s)" % want in plan.describe(), plan.describe()
+            plan.execute(to_dev(x).data_ptr(), y.data_ptr())
+            got = y.cpu().numpy()
+            ref = oracle.c2c(gather(x, hm, d, n, s).astype(np.complex128), -1)
+            assert oracle.rel_l2(gather(got, hm, d, n, s), ref) <= oracle.fp32_tol(n), plan.describe()
+            touched = np.zeros(got.size, bool)
+            touched[(np.arange(hm)[:, None] * d + np.arange(n)[None, :] * s).ravel()] = True
+            assert np.all(got[~touched] == 7.0), "wrote outside the members"
+
+
 # n <= 4096 (one pass), one-buffer and two-buffer tiles, a two-pass length;
 # 2^-53 per rounding, 8 log2 n of them
 @pytest.mark.parametrize("n", [2, 13, 64, 143, 1000, 2048, 4096, 5000, 8192, 30000])
@@ -78,7 +100,7 @@ def test_c2c_fp16(n, offset, strided):
     assert oracle.rel_l2(gather(got, hm, d, n, s), ref) <= 2.0**-11 + oracle.fp32_tol(n), plan.describe()
 
 
-REAL_LENGTHS = [4, 6, 26, 32, 100, 242, 1000, 2002, 4374, 8000, 20000]
+REAL_LENGTHS = [4, 6, 26, 28, 30, 32, 100, 242, 1000, 2002, 4374, 8000, 20000]
 R2R = [plfft.R2RKind.DCT_2, plfft.R2RKind.DCT_3, plfft.R2RKind.DCT_4, plfft.R2RKind.DST_2, plfft.R2RKind.DST_3,
        plfft.R2RKind.DST_4, plfft.R2RKind.DHT, plfft.R2RKind.R2HC, plfft.R2RKind.HC2R]
 
@@ -105,7 +127,7 @@ def test_r2c_c2r(n, pad):
         assert np.all(got[np.arange(hm - 1) * (n + 1) + n] == 7.0), "wrote between the members"
 
 
-@pytest.mark.parametrize("n", [6, 26, 100, 1000, 2002])
+@pytest.mark.parametrize("n", [6, 26, 28, 30, 32, 100, 1000, 2002])
 @pytest.mark.parametrize("kind", R2R)
 def test_r2r(n, kind):
     import torch
