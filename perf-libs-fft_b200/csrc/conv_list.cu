@@ -16,6 +16,7 @@ cudaError_t launch_conv_list_bluestein(int m, const ConvFusedLaunch& P, cudaStre
 //   640: 98 / 100 (n=317)    768: 89 / 97 (n=383)
 //   1152: 107 / 131 (n=577, Rader)   1280: 107 / 121 (n=641, Rader)   1536: 90 / 105 (n=761)
 //   2304: 104 / 148 (n=1031)   2560: 96 / 125 (n=1279)   3072: 104 / 110 (n=1531)
+// and for some only up to or from a batch (the rule in plan_conv.cpp).
 // Not listed: 320 to 448 (132 / 125), 896 (108 / 86), 1408 and 2816 (even),
 // 1664 (128 / 105), 1792, 3328, 3584 and 3840, whose larger or prime first
 // radix or length eats the gain.

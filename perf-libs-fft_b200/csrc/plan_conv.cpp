@@ -313,6 +313,21 @@ static std::unique_ptr<Node> make_conv_list(int64_t n, const Layout& lay, int di
   if (l.empty()) return nullptr;
   const int64_t m = int64_t(l[0]) * l[1] * l[2], p2 = conv_fused_length(n);
   if (m > p2) return nullptr;
+  // What the shorter length saves against its longer chain of stages, us for
+  // 1 / 148 / 1024 / 2048 members and 2^23 numbers, power of two first:
+  //   640:  Rader n=313 8.3 7.3, 10.3 7.8, 10.3 10.0, 12.4 17.9, 105 122;
+  //         Bluestein n=277 6.2 5.2, 7.6 5.7, 8.3 7.6, 12.4 14.5, 107 110
+  //   768:  Rader n=353 8.3 6.1, 10.3 6.5, 10.4 9.0, 12.9 16.5, 102 118;
+  //         Bluestein n=383 6.2 5.6, 8.3 6.1, 9.1 8.1, 12.9 14.1, 98 89
+  //   1280: Rader n=601 6.2 6.6, 6.2 7.2, 14.4 16.4, 22.6 21.5, 127 116;
+  //         Bluestein n=593 6.2 5.8, 6.2 6.2, 13.4 14.6, 22.6 18.6, 129 98
+  // and from 1536 up both gain, or lose 8 % at most at single batches.
+  const int64_t hm = lay.howmany;
+  if (m == 640 || (m == 768 && rader)) {
+    if (hm > 1024) return nullptr;
+  } else if (m < 1536 && rader && hm <= 148) {
+    return nullptr;
+  }
   auto node = std::make_unique<ConvFusedNode>();
   node->rader = rader;
   node->list = true;

@@ -251,3 +251,19 @@ def test_conv_list(n, direction):
             ref = oracle.c2c(gather(x, hm, d, n, s).astype(np.complex128), direction, method="fft")
             got = gather(y.cpu().numpy(), hm, d, n, s)
             assert oracle.rel_l2(got, ref) <= oracle.fp32_tol(n), plan.describe()
+
+
+# which of them a batch takes: the ends of each rule
+@pytest.mark.parametrize("n,hm,listed", [(313, 1024, True), (313, 1025, False), (277, 1025, False), (331, 1024, True),
+                                         (331, 1025, False), (383, 1025, True), (521, 148, False), (521, 149, True),
+                                         (601, 149, True), (641, 149, True), (563, 3, True), (677, 3, True)])
+def test_conv_list_batches(n, hm, listed):
+    import torch
+
+    x = seeded_complex(hm * n, n)
+    y = torch.zeros(x.size, dtype=torch.complex64, device="cuda")
+    plan = plfft.make_plan("c2c", n, hm)
+    assert (" list)" in plan.describe()) == listed, plan.describe()
+    plan.execute(to_dev(x).data_ptr(), y.data_ptr())
+    ref = oracle.c2c(x.reshape(hm, n).astype(np.complex128), -1, method="fft")
+    assert oracle.rel_l2(y.cpu().numpy().reshape(hm, n), ref) <= oracle.fp32_tol(n), plan.describe()
