@@ -267,3 +267,18 @@ def test_conv_list_batches(n, hm, listed):
     plan.execute(to_dev(x).data_ptr(), y.data_ptr())
     ref = oracle.c2c(x.reshape(hm, n).astype(np.complex128), -1, method="fft")
     assert oracle.rel_l2(y.cpu().numpy().reshape(hm, n), ref) <= oracle.fp32_tol(n), plan.describe()
+
+
+# short lengths of 11 and 13 in small batches: direct sums
+@pytest.mark.parametrize("n,hm,sums", [(11, 1000, True), (11, 1001, False), (26, 7, True), (26, 1001, False), (33, 7, False)])
+def test_fp64_short(n, hm, sums):
+    import torch
+
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-1, 1, n * hm) + 1j * rng.uniform(-1, 1, n * hm)
+    y = torch.zeros(n * hm, dtype=torch.complex128, device="cuda")
+    plan = plfft.make_plan("c2c", n, hm, data_type=plfft.DataType.FP64)
+    assert ("direct sums" in plan.describe()) == sums, plan.describe()
+    plan.execute(to_dev(x).data_ptr(), y.data_ptr())
+    tol = 8 * np.log2(n) * 2.0**-53
+    assert oracle.rel_l2(y.cpu().numpy().reshape(hm, n), np.fft.fft(x.reshape(hm, n))) <= tol, plan.describe()
