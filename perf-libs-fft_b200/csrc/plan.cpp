@@ -844,6 +844,26 @@ std::unique_ptr<Node> make_c2c_node(int64_t n, const Layout& lay, int dir, float
   return make_conv_node(n, lay, dir, scale, why);
 }
 
+// A few small transforms between other kernels: the tile kernel, whose code
+// is shorter, than the mixed-radix engine, which pays when its code is in the
+// SM's instruction cache (that is, back to back).  R2C of odd n in a graph, us,
+// tile / engine: n=33 x 1 6.6 / 8.9, n=225 x 1 8.4 / 12.7, n=39 x 8 7.0 / 10.0,
+// n=891 x 1 11.0 / 11.1, n=27 x 64 11.8 / 9.5; of 11 and 13 up to more
+// elements: n=65 x 64 10.5 / 12.7, n=363 x 8 11.6 / 12.1, n=847 x 8 equal.
+// Convolutions likewise: over the power of two (DCT-I of 363 x 1..64, inner
+// length 724, 7.5..8.4, and 9.0..10.2 over 1536 points).
+std::unique_ptr<Node> make_c2c_inner_node(int64_t n, const Layout& lay, int dir, float scale, std::string* why) {
+  const int64_t top = n % 11 == 0 || n % 13 == 0 ? 4224 : 960;
+  const bool pow2 = is_pow2(n) && n >= 64;
+  if (n > 8 && !pow2 && is_smooth(n) && n * lay.howmany <= top && lay.istride == 1 && lay.ostride == 1) {
+    Addr ia{lay.idist, 0, 1, 1}, oa{lay.odist, 0, 1, 1};
+    if (auto t = make_tile(n, lay.howmany, ia, oa, dir, scale, false, why)) return t;
+  }
+  if (!is_smooth(n) && conv_fused_length(n) && lay.howmany <= 64)
+    if (auto c = make_conv_fused(n, lay, dir, scale, why, -1, 0, 0)) return c;
+  return make_c2c_node(n, lay, dir, scale, 0, why);
+}
+
 // Alternative schedules for the same C2C problem, default first (the
 // autotuner times them).  level 1: launch shapes of the chosen kernel
 // family; level 2: also other kernel families and radix sizes; level 3:

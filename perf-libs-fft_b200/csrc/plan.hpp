@@ -159,6 +159,9 @@ int64_t four_step_split(int64_t n);
 std::unique_ptr<Node> make_c2c_node(int64_t n, const Layout& lay, int dir, float scale,
                                     int precision, std::string* why);
 
+// The same between a real transform's own elementwise launches.
+std::unique_ptr<Node> make_c2c_inner_node(int64_t n, const Layout& lay, int dir, float scale, std::string* why);
+
 // Alternative C2C schedules for the autotuner, the default first; level 1-3
 // widens the search (launch shapes, kernel families, four-step shapes).
 std::vector<std::unique_ptr<Node>> make_c2c_candidates(int64_t n, const Layout& lay, int dir, float scale,

@@ -192,8 +192,8 @@ std::unique_ptr<Node> make_realwrap_node(int kind, int64_t n, const Layout& lay,
   auto inner_for = [&](int64_t count) {
     // R2C: pairs of the input (complex distance idist / 2) into work; C2R:
     // work into pairs of the output (odist / 2), with the plan's scale
-    return node->r2c ? make_c2c_node(m, Layout{count, 1, lay.idist / 2, 1, m}, -1, 1.0f, 0, why)
-                     : make_c2c_node(m, Layout{count, 1, m, 1, lay.odist / 2}, +1, float(scale), 0, why);
+    return node->r2c ? make_c2c_inner_node(m, Layout{count, 1, lay.idist / 2, 1, m}, -1, 1.0f, why)
+                     : make_c2c_inner_node(m, Layout{count, 1, m, 1, lay.odist / 2}, +1, float(scale), why);
   };
   node->inner = inner_for(node->chunk);
   if (!node->inner) return nullptr;
@@ -235,7 +235,7 @@ static std::unique_ptr<Node> make_realwrap_generic(int kind, int64_t n, const La
   node->chunk = std::max<int64_t>(1, std::min<int64_t>(lay.howmany, target / (node->len * int64_t(node->cbytes()))));
   Layout inner{node->chunk, 1, node->len, 1, node->len};
   node->inner = fp64 ? make_fp64_c2c(node->len, inner, wrap_dir(kind), 1.0, why)
-                     : make_c2c_node(node->len, inner, wrap_dir(kind), 1.0f, 0, why);
+                     : make_c2c_inner_node(node->len, inner, wrap_dir(kind), 1.0f, why);
   if (!node->inner) return nullptr;
   return node;
 }

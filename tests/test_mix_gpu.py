@@ -282,3 +282,21 @@ def test_fp64_short(n, hm, sums):
     plan.execute(to_dev(x).data_ptr(), y.data_ptr())
     tol = 8 * np.log2(n) * 2.0**-53
     assert oracle.rel_l2(y.cpu().numpy().reshape(hm, n), np.fft.fft(x.reshape(hm, n))) <= tol, plan.describe()
+
+
+# small batches inside a real transform: the tile kernel and the power-of-two
+# convolution
+@pytest.mark.parametrize("n,hm,inner", [(9, 106, "c2c-tile"), (9, 107, "c2c-mix"), (33, 128, "c2c-tile"), (33, 129, "c2c-mix"),
+                                        (1001, 4, "c2c-tile"), (1001, 5, "c2c-mix"), (17, 64, "e="), (1031, 64, "m=4096"),
+                                        (1031, 65, "m=2304")])
+def test_real_small_batches(n, hm, inner):
+    import torch
+
+    h = n // 2 + 1
+    x = seeded_real(hm * n, n)
+    y = torch.zeros(hm * h, dtype=torch.complex64, device="cuda")
+    plan = plfft.make_plan("r2c", n, hm)
+    assert inner in plan.describe(), plan.describe()
+    plan.execute(to_dev(x).data_ptr(), y.data_ptr())
+    ref = np.fft.rfft(x.reshape(hm, n).astype(np.float64))
+    assert oracle.rel_l2(y.cpu().numpy().reshape(hm, h), ref) <= oracle.fp32_tol(n), plan.describe()
