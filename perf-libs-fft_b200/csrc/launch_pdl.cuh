@@ -21,20 +21,32 @@ inline bool pdl_enabled() {
   return on;
 }
 
+// carveout: percent of an SM's memory to be shared memory, 0 for the driver's
+// choice by the kernel's occupancy
 template <class... Params, class... Args>
-cudaError_t launch_pdl(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                       Args&&... args) {
+cudaError_t launch_pdl_carved(int carveout, void (*kern)(Params...), dim3 grid, dim3 block, size_t smem,
+                              cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  if (carveout) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[cfg.numAttrs++].val.sharedMemCarveout = unsigned(carveout);
+  }
   return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
+template <class... Params, class... Args>
+cudaError_t launch_pdl(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                       Args&&... args) {
+  return launch_pdl_carved(0, kern, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 }  // namespace plfft_b200

@@ -101,7 +101,7 @@ struct MixIoF64 {
 
 // FP32 arithmetic on sequences of type U, two sequences (2 c and 2 c + 1) per engine element; an odd
 // last sequence rides alone, its partner a copy that is not stored
-template <class U, int DIR>
+template <class U, int DIR, bool BY_MEMBER = false>
 struct MixIoPair {
   const U* in;
   U* out;
@@ -121,7 +121,7 @@ struct MixIoPair {
     oks = L.oa.kstride;
     scale = float(L.scale);
     post = L.post;
-    col0 = uint32_t(col);
+    col0 = uint32_t(BY_MEMBER ? m : col);
     const int64_t left = L.ncols - col;
     count = left < 2 * L.d.c ? int(left) : 2 * L.d.c;
     wide_in = L.wide_in;
@@ -161,8 +161,9 @@ struct MixIoPair {
   }
   __device__ __forceinline__ cpair finish(cpair y, int c, int k) const {
     if (post.lo) {
-      const uint32_t col = col0 + 2u * uint32_t(c);
-      const cpair w = join(twiddle(col * uint32_t(k)), twiddle((col + (2 * c + 1 < count)) * uint32_t(k)));
+      const uint32_t col = BY_MEMBER ? col0 : col0 + 2u * uint32_t(c);
+      const cpair w = join(twiddle(col * uint32_t(k)),
+                           twiddle((BY_MEMBER ? col : col + (2 * c + 1 < count)) * uint32_t(k)));
       const float2 wi = DIR < 0 ? w.im : fneg2(w.im);
       y = cpair{__ffma2_rn(y.im, fneg2(wi), __fmul2_rn(y.re, w.re)), __ffma2_rn(y.im, w.re, __fmul2_rn(y.re, wi))};
     }
@@ -361,7 +362,7 @@ cudaError_t run_mix(const MixLaunch<typename MixTraits<V>::W>& L, cudaStream_t s
   if (e != cudaSuccess) return e;
   const int64_t grid = L.members * int64_t(L.tpm);
   if (grid > 0x7fffffff) return cudaErrorInvalidValue;
-  return launch_pdl(k, dim3(unsigned(grid)), dim3(L.d.nthr), size_t(smem), st, L);
+  return launch_pdl_carved(L.carveout, k, dim3(unsigned(grid)), dim3(L.d.nthr), size_t(smem), st, L);
 }
 
 }  // namespace plfft_b200

@@ -48,7 +48,8 @@ struct MixAddr {
   int64_t mdist, cdist, kstride;
 };
 
-// two-level four-step twiddle W_N^e = lo[e mod 2^shift] * hi[e >> shift]
+// two-level four-step twiddle W_N^e = lo[e mod 2^shift] * hi[e >> shift] on
+// output k: e = column * k
 template <class W>
 struct MixPost {
   const W* lo;
@@ -69,6 +70,7 @@ struct MixLaunch {
   double scale;
   const W* tw;
   MixPost<W> post;  // lo == nullptr: none
+  int carveout = 0;  // share of shared memory, percent (0: the driver's choice)
   MixDesc d;
 };
 
@@ -92,6 +94,8 @@ cudaError_t launch_mix_real(int kind, const MixRealLaunch& L, cudaStream_t st);
 
 int mix_smem_bytes(const MixDesc& d);
 cudaError_t launch_mix_f32(int dir, const MixLaunch<float2>& L, cudaStream_t st);
+// the post twiddle goes by member, not by column
+cudaError_t launch_mix_f32_members(int dir, const MixLaunch<float2>& L, cudaStream_t st);
 // binary16 buffers; pairs: both aligned for 4-byte (re, im) accesses
 cudaError_t launch_mix_f16(int dir, bool pairs, const MixLaunch<float2>& L, cudaStream_t st);
 cudaError_t launch_mix_f16_scalar(int dir, const MixLaunch<float2>& L, cudaStream_t st);

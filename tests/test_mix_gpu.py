@@ -300,3 +300,27 @@ def test_real_small_batches(n, hm, inner):
     plan.execute(to_dev(x).data_ptr(), y.data_ptr())
     ref = np.fft.rfft(x.reshape(hm, n).astype(np.float64))
     assert oracle.rel_l2(y.cpu().numpy().reshape(hm, h), ref) <= oracle.fp32_tol(n), plan.describe()
+
+
+# two passes over interleaved members: lanes along the members from eight of
+# them, a short last chunk (600000 x 23), an odd pitch, in place, one side dense
+@pytest.mark.parametrize("n,hm", [(12000, 7), (12000, 8), (13312, 37), (16250, 64), (600000, 23)])
+@pytest.mark.parametrize("direction", [-1, 1])
+def test_four_step_members(n, hm, direction):
+    import torch
+
+    for i, o in [((hm, 1), (hm, 1)), ((hm + 1, 1), (hm + 2, 1)), ((1, n), (hm, 1))]:
+        x = torch.randn(span(hm, i[1], n, i[0]), dtype=torch.complex64, device="cuda",
+                        generator=torch.Generator("cuda").manual_seed(n))
+        plan = plfft.make_plan("c2c", n, hm, *i, *o, direction=direction, alias=plfft.IoAlias.MAY_ALIAS, scale=0.5)
+        assert ("member lanes" in plan.describe()) == (hm >= 8 and i[0] > 1), plan.describe()
+        y = torch.full((span(hm, o[1], n, o[0]),), 7.0, dtype=torch.complex64, device="cuda")
+        xl = torch.as_strided(x, (hm, n), (i[1], i[0])).to(torch.complex128)
+        ref = 0.5 * (torch.fft.fft(xl) if direction < 0 else torch.fft.ifft(xl) * n)
+        for dst in (y, x) if i == o else (y,):  # the second: in place
+            plan.execute(x.data_ptr(), dst.data_ptr())
+            got = torch.as_strided(dst, (hm, n), (o[1], o[0]))
+            assert float((got - ref).norm() / ref.norm()) <= oracle.fp32_tol(n), plan.describe()
+        untouched = torch.ones(y.numel(), dtype=torch.bool, device="cuda")
+        torch.as_strided(untouched, (hm, n), (o[1], o[0])).fill_(False)
+        assert bool((y[untouched] == 7.0).all()), "wrote outside the members"
