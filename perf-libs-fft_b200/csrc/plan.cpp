@@ -863,6 +863,13 @@ std::unique_ptr<Node> make_c2c_node(int64_t n, const Layout& lay, int dir, float
     auto p2 = make_pow2(n, lay, dir, scale, why);
     if (p2) return p2;
   }
+  // one to four members of a length with radix 11 or 13: the tile kernel ends
+  // sooner (us, tile / engine, back to back n=847 x 1 5.2 / 6.0, after another
+  // kernel 6.6 / 8.3, n=169 x 4 5.7 / 7.6, n=1040 x 1 7.0 / 7.6, x 8 equal)
+  if (unit && lay.howmany <= 4 && n <= 1040 && is_smooth(n) && (n % 11 == 0 || n % 13 == 0)) {
+    Addr ia{lay.idist, 0, 1, 1}, oa{lay.odist, 0, 1, 1};
+    if (auto t = make_tile(n, lay.howmany, ia, oa, dir, scale, false, why)) return t;
+  }
   // dense powers of two beyond the on-chip kernel keep the bulk-copy four-step
   if (!(unit && is_pow2(n) && n > 8192))
     if (auto t = make_mix_c2c<float2>(n, lay, dir, scale, false, why)) return t;

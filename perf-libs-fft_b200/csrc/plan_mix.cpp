@@ -204,8 +204,9 @@ bool mix_shape(MixDesc& d, int64_t n, int64_t count, bool cf_in, bool cf_out, in
   // more a dense side pays for lanes that lie n elements apart: two stages
   // (us, 2^22 numbers, one / two: C2C n=14 22.6 / 19.8, 15 23.3 / 15.7, 16
   // 28.2 / 16.8; C2R n=32 47.0 / 13.0; n=12 19.3 / 16.1, but its real kinds
-  // of 1000 members 4.3 / 5.6).
-  if (n >= 14 && radices.size() == 1 && !(cf_in && cf_out)) radices = mix_radices(n, int(n) - 1);
+  // of 1000 members 4.3 / 5.6).  Few members end sooner in one (C2C n=16 x 4
+  // after another kernel 4.0 / 4.8, x 1000 4.9 / 4.3).
+  if (n >= 14 && count > 128 && radices.size() == 1 && !(cf_in && cf_out)) radices = mix_radices(n, int(n) - 1);
   MixDesc best{};
   double best_cost = -1;
   // strided batches move segments of c consecutive elements: whole 32-byte

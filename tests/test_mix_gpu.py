@@ -270,7 +270,8 @@ def test_conv_list_batches(n, hm, listed):
 
 
 # short lengths of 11 and 13 in small batches: direct sums
-@pytest.mark.parametrize("n,hm,sums", [(11, 1000, True), (11, 1001, False), (26, 7, True), (26, 1001, False), (33, 7, False)])
+@pytest.mark.parametrize("n,hm,sums", [(11, 1000, True), (11, 1001, False), (26, 7, True), (26, 1001, False),
+                                       (33, 256, True), (39, 257, False), (44, 7, False)])
 def test_fp64_short(n, hm, sums):
     import torch
 
@@ -324,3 +325,18 @@ def test_four_step_members(n, hm, direction):
         untouched = torch.ones(y.numel(), dtype=torch.bool, device="cuda")
         torch.as_strided(untouched, (hm, n), (o[1], o[0])).fill_(False)
         assert bool((y[untouched] == 7.0).all()), "wrote outside the members"
+
+
+# one to four members of lengths with radix 11 or 13
+@pytest.mark.parametrize("n,hm,tile", [(11, 4, True), (169, 1, True), (242, 4, True), (242, 5, False), (1040, 3, True),
+                                       (1001, 5, False), (1053, 1, False), (1000, 1, False)])
+def test_few_members(n, hm, tile):
+    import torch
+
+    x = seeded_complex(hm * n, n)
+    y = torch.zeros(x.size, dtype=torch.complex64, device="cuda")
+    plan = plfft.make_plan("c2c", n, hm)
+    assert ("c2c-tile" in plan.describe()) == tile, plan.describe()
+    plan.execute(to_dev(x).data_ptr(), y.data_ptr())
+    ref = oracle.c2c(x.reshape(hm, n).astype(np.complex128), -1)
+    assert oracle.rel_l2(y.cpu().numpy().reshape(hm, n), ref) <= oracle.fp32_tol(n), plan.describe()
