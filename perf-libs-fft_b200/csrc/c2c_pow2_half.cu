@@ -3,8 +3,9 @@
 // user's buffers, one launch and 8 bytes of HBM traffic per element.
 //
 // T = N/E threads per transform, whole warps' worth of transforms per CTA.
-// Bound by latency like its FP32 sibling, at half the bytes.  Forward and back,
-// N=1024 x 4096 each: see the figure at the dispatch in plan_mix.cpp.
+// Bound by latency like its FP32 sibling, at half the bytes: 108 registers at
+// N=1024 leave four 128-thread CTAs to an SM, 1.7 waves of the 1024 of a
+// 4096-member batch.  Figures of both sides at the dispatch in plan_mix.cpp.
 #include "kernels.h"
 #include "launch_pdl.cuh"
 #include "pow2_stages.cuh"
@@ -78,17 +79,22 @@ static cudaError_t run_half(int dir, Pow2HalfLaunch L, cudaStream_t st) {
   return launch_pdl(k, dim3(unsigned(grid)), dim3(T * L.g), size_t(smem), st, L);
 }
 
-int pow2_half_e(int64_t n) { return n == 64 ? 8 : n == 1024 || n == 2048 || n == 8192 ? 32 : 16; }
+// Elements per thread, us at 2^24 numbers a call with 8 / 16 / 32:
+//   64: 36.7 / 46.6 / 80.4     128: 36.4 / 35.2 / 47.3    256: 32.8 / 23.7 / 35.5
+//   512: 36.0 / 31.9 / 26.6    1024: 48.6 / 34.5 / 27.7   2048: 64.5 / 35.3 / 38.7
+//   4096: 82.5 / 43.0 / 39.5   8192: - / 71.3 / 47.5
+// (2^22 numbers order them alike.)
+int pow2_half_e(int64_t n) { return n == 64 ? 8 : n == 128 || n == 256 || n == 2048 ? 16 : 32; }
 
 cudaError_t launch_c2c_pow2_half(int n, int dir, const Pow2HalfLaunch& L, cudaStream_t st) {
   switch (n) {
     case 64: return run_half<64, 8>(dir, L, st);
     case 128: return run_half<128, 16>(dir, L, st);
     case 256: return run_half<256, 16>(dir, L, st);
-    case 512: return run_half<512, 16>(dir, L, st);
+    case 512: return run_half<512, 32>(dir, L, st);
     case 1024: return run_half<1024, 32>(dir, L, st);
-    case 2048: return run_half<2048, 32>(dir, L, st);
-    case 4096: return run_half<4096, 16>(dir, L, st);
+    case 2048: return run_half<2048, 16>(dir, L, st);
+    case 4096: return run_half<4096, 32>(dir, L, st);
     case 8192: return run_half<8192, 32>(dir, L, st);
     default: return cudaErrorInvalidValue;
   }
