@@ -10,8 +10,9 @@ from helpers import gather, seeded_complex, seeded_real, span, to_dev
 pytestmark = pytest.mark.gpu
 
 # one stage (2, 13, 16), two, three, four; primes of the radix menu; a tile of
-# many transforms and of one; the longest one- and two-buffer tiles
-LENGTHS = [2, 13, 16, 18, 121, 169, 210, 360, 1000, 1001, 1155, 2187, 4000, 6561, 8000, 12000, 14336]
+# many transforms and of one; the longest two- and one-buffer tiles (7128, 8788);
+# 8000 and beyond: the tile kernel or two passes
+LENGTHS = [2, 13, 16, 18, 121, 169, 210, 360, 1000, 1001, 1155, 2187, 4000, 6561, 7128, 8000, 8788, 12000, 14336]
 
 
 @pytest.mark.parametrize("n", LENGTHS)
@@ -32,6 +33,59 @@ def test_c2c_fp32(n, direction):
         touched = np.zeros(got.size, bool)
         touched[(np.arange(hm)[:, None] * od + np.arange(n)[None, :] * os_).ravel()] = True
         assert np.all(got[~touched] == 7.0), "wrote outside the members"
+
+
+# which of them the engine holds in one pass
+@pytest.mark.parametrize("n,buffers", [(4095, "one-buffer"), (6561, ""), (7128, "two-buffers"), (8788, "one-buffer"),
+                                       (6720, None), (8000, None), (8190, None)])
+def test_c2c_reach(n, buffers):
+    d = plfft.make_plan("c2c", n, 37).describe()
+    assert d.startswith("(c2c-mix") == (buffers is not None) and (not buffers or buffers in d), d
+
+
+# members interleaved at an even pitch: two numbers to an aligned 16-byte word,
+# an odd last member, the same bases one element further, and in place
+@pytest.mark.parametrize("n", [2, 13, 16, 30, 169, 1000, 4095])
+@pytest.mark.parametrize("pitch,hm", [(38, 37), (40, 37), (2, 2), (4, 3)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_c2c_fp32_pairs(n, pitch, hm, offset):
+    import torch
+
+    m = span(hm, 1, n, pitch)
+    x = seeded_complex(m + offset, n)
+    plan = plfft.make_plan("c2c", n, hm, pitch, 1, pitch, 1, alias=plfft.IoAlias.MAY_ALIAS)
+    ref = oracle.c2c(gather(x[offset:], hm, 1, n, pitch).astype(np.complex128), -1, method="fft" if n > 16 else "auto")
+    touched = np.zeros(m + offset, bool)
+    touched[offset + (np.arange(hm)[:, None] + np.arange(n)[None, :] * pitch).ravel()] = True
+    d = to_dev(x)
+    for dst in (torch.full((m + offset + 2,), 7.0, dtype=torch.complex64, device="cuda"), d):
+        before = dst.cpu().numpy()[: m + offset]
+        plan.execute(d.data_ptr() + 8 * offset, dst.data_ptr() + 8 * offset)
+        got = dst.cpu().numpy()
+        assert oracle.rel_l2(gather(got[offset:], hm, 1, n, pitch), ref) <= oracle.fp32_tol(n), plan.describe()
+        assert np.array_equal(got[: m + offset][~touched], before[~touched]), "wrote outside the members"
+        assert np.all(got[m + offset:] == 7.0), "wrote behind the members"
+
+
+# in place with equal layouts, dense and interleaved, several CTAs
+@pytest.mark.parametrize("n,hm", [(18, 5001), (1000, 301), (4095, 37), (8788, 5)])
+@pytest.mark.parametrize("dense", [True, False])
+@pytest.mark.parametrize("kind", ["FP32", "FP64", "FP16"])
+def test_c2c_in_place(n, hm, dense, kind):
+    if (kind == "FP64" and n == 8788) or (kind == "FP16" and n > 4096):
+        n = 7168 if kind == "FP64" else 4000
+    s, d = (1, n) if dense else (hm, 1)
+    rng = np.random.default_rng(n)
+    real = {"FP32": np.float32, "FP64": np.float64, "FP16": np.float16}[kind]
+    x = rng.uniform(-1, 1, 2 * n * hm).astype(real)
+    plan = plfft.make_plan("c2c", n, hm, s, d, s, d, data_type=plfft.DataType[kind], scale=n**-0.5,
+                           alias=plfft.IoAlias.MAY_ALIAS)
+    buf = to_dev(x)
+    plan.execute(buf.data_ptr(), buf.data_ptr())
+    z = gather(x.astype(np.float64).view(np.complex128), hm, d, n, s)
+    got = gather(buf.cpu().numpy().astype(np.float64).view(np.complex128), hm, d, n, s)
+    tol = {"FP32": oracle.fp32_tol(n), "FP64": 8 * np.log2(n) * 2.0**-53, "FP16": 2.0**-11 + oracle.fp32_tol(n)}[kind]
+    assert oracle.rel_l2(got, np.fft.fft(z) * n**-0.5) <= tol, plan.describe()
 
 
 # lengths of one radix: stored from shared memory, or from 14 points on a dense
