@@ -112,7 +112,7 @@ plfft_status_t plfft_cuda_group_execute_async(plfft_cuda_group_t *group,
  * 192-201 semantics).  PLFFT_ESTIMATE is plfft_cuda_group_create (its
  * default schedule).  MEASURE, PATIENT and EXHAUSTIVE build candidate
  * schedules of the group (four-step tile width, same-length transforms
- * merged into one task, largest radix; 4, 6 and 10 candidates), time each on scratch device buffers of the
+ * merged into one task, largest radix; 3, 4 and 7 candidates), time each on scratch device buffers of the
  * group's spans within 0.1 / 0.5 / 2 s of timed work, keep the fastest and
  * remember it in the wisdom (plfft_cuda_wisdom_*), keyed by the lengths,
  * offsets, direction and device.  Returns PLFFT_INVALID_PLANNER_RIGOR for

@@ -28,8 +28,9 @@ namespace plfft_b200 {
 // with the stage list of the task in shared memory.  256 threads at 64
 // registers and 36 KB of tile, four CTAs per SM: while some tiles wait for
 // their loads or at a barrier the others compute (two CTAs of 512 threads
-// took 807 us on the 4000-transform mix, these 727), and 16 four-step columns of 256 are
-// whole 128-byte segments.
+// took 807 us on the 4000-transform mix, these 727, and 659 with the lengths
+// and splits that grouped_plan.cpp chooses by cost), and 16 four-step columns
+// of 256 are whole 128-byte segments.
 constexpr int kGroupThreads = 256, kGroupPerSm = 4;
 
 __device__ __forceinline__ float2 group_conj(float2 v, bool on) { return on ? make_float2(v.x, -v.y) : v; }

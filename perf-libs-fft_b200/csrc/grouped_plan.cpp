@@ -46,10 +46,11 @@ struct Tables {
 
 // Schedule of a grouped execution (the autotuner's choices): columns or rows
 // per four-step tile, same-length on-chip transforms merged into one task,
-// largest radix of the on-chip stage lists.
+// largest radix of the on-chip stage lists (16 at most).
 struct GroupShape {
-  // measured on the 4000-transform mix: 32-wide tiles 1.15x over 16, 8 at
-  // 0.77x; merging 1.02x; radix 8 or 32 below 16
+  // measured on the 4000-transform mix, us: tiles up to 8 / 16 / 24 / 32 / 64
+  // wide 901 / 703 / 683 / 658 / 661 (no length above 144 fills 32); merging
+  // up to 1 / 4 / 16 / 64 transforms 681 / 666 / 658 / 658; radix 8 801
   int tile_cap = 32;
   int merge_cap = 16;
   int max_radix = 16;
@@ -717,19 +718,15 @@ plfft_status_t plfft_cuda_group_create_tuned(plfft_cuda_group_t** group, int64_t
     sh.max_radix = radix;
     cands.push_back(sh);
   };
+  // (wider tiles than 32 and larger radices than 16 give the first again)
   add(32, 16, 16);
   add(16, 16, 16);
-  add(64, 16, 16);
   add(32, 1, 16);
-  if (rigor >= PLFFT_PATIENT) {
-    add(32, 16, 8);
-    add(32, 16, 32);
-  }
+  if (rigor >= PLFFT_PATIENT) add(32, 16, 8);
   if (rigor >= PLFFT_EXHAUSTIVE) {
     add(8, 16, 16);
     add(16, 1, 16);
     add(32, 64, 16);
-    add(64, 64, 16);
   }
   // the problem's key: FNV-1a over lengths and offsets, the count, direction, device
   uint64_t hsh = 1469598103934665603ull;

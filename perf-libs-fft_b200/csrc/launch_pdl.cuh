@@ -3,8 +3,9 @@
 // A kernel launched this way may have its CTAs placed on SMs while the
 // previous kernel in the stream drains, so launch latency and the kernel's
 // own set-up overlap that kernel's last CTAs.  Every kernel launched through
-// launch_pdl calls griddep_wait() (ptx.cuh) before its first global read or
-// write, which holds it until the previous kernel has completed and its
+// launch_pdl calls griddep_wait() (ptx.cuh) before its first access to memory
+// that a kernel may write (tables of the plan, which none writes, may be read
+// earlier), which holds it until the previous kernel has completed and its
 // writes are visible: stream order is unchanged for the data.
 // PLFFT_B200_NO_PDL=1 launches without the attribute.
 #pragma once

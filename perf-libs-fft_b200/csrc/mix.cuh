@@ -10,9 +10,9 @@
 // twiddle loads and operand moves per number), 80 registers and one exchange
 // buffer.  C2C N=1000 x 16384 (262 MB): 149 us through the tile kernel of
 // c2c.cu, 78 us with single FP32 numbers at 64 registers, 74 us with pairs at
-// 128 registers and two buffers, 63 us as it is (4.1 TB/s).  Copying the next
-// tile ahead into shared memory cost more shared-memory traffic than it hid
-// (92 us) and was not kept.
+// 128 registers and two buffers, 63 us as it is (4.1 TB/s; 66.6 us with other
+// inputs on each pass).  Copying the next tile ahead into shared memory cost
+// more shared-memory traffic than it hid (92 us) and was not kept.
 #pragma once
 #include <cuda_fp16.h>
 

@@ -32,8 +32,7 @@ bool is_smooth(int64_t n) {
 // Split n into radices <= max_radix, largest first.  Mirrors the intent of
 // the reference's factorize_descending (src/factorize.hpp:95-111): greedy
 // division by the largest available kernel size.  The radix menu here is the
-// set of on-chip codelets {16, 8, 4, 2, 13, 11, 7, 5, 3} (32 in the register
-// engine).
+// set of on-chip codelets {16, 8, 4, 2, 13, 11, 7, 5, 3}.
 std::vector<int> factor_radices(int64_t n, int max_radix) {
   std::vector<int> r;
   const int pow2_menu[] = {32, 16, 8, 4, 2};

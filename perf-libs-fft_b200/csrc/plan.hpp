@@ -213,8 +213,9 @@ std::unique_ptr<Node> make_realwrap_node(int kind, int64_t n, const Layout& lay,
 // schedule.
 std::unique_ptr<Node> make_fp64_c2c(int64_t n, const Layout& lay, int dir, double scale, std::string* why);
 
-// One-kernel R2C / C2R / DCT-II / DST-II (FusedRealKind) for N = 2M, M a
-// power of two in [64, 8192], unit strides; nullptr when not applicable.
+// One-kernel real transforms (FusedRealKind) for N = 2M, unit strides: M a power
+// of two in [64, 8192] (real_fused.cu) or another smooth length that the
+// mixed-radix tiles hold (mix_real.cu); nullptr when not applicable.
 // wmode: adjoint weights (RealFusedLaunch::wmode), 0 for the plain transform.
 std::unique_ptr<Node> make_real_fused_node(int kind, int64_t n, const Layout& lay, float scale, int wmode = 0,
                                            int g_override = 0, int e_override = 0);

@@ -150,6 +150,17 @@ static void mix_set_tile(MixDesc& d, int c) {
 
 namespace {
 
+int sm_count() {
+  static const int n = [] {
+    int dev = 0, sms = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+                   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0
+               ? sms
+               : 148;  // no device here (the planner's own tests)
+  }();
+  return n;
+}
+
 // shared memory of an SM that tiles may fill, and of one CTA
 constexpr int kSmemPerSm = 227 * 1024, kSmemPerCta = 224 * 1024;
 // Estimated time of a shape per element, in issued instructions: every
@@ -186,7 +197,7 @@ double shape_cost(const MixDesc& d, int64_t ncols, int lanes) {
   // (N=500 x 32768: 59.5 us with one buffer, 71 with two)
   if (!d.inplace) cost *= 1.12;
   // too few tiles for the chip: the tile's own latency counts
-  const double waves = double(tiles) / (148.0 * per_sm);
+  const double waves = double(tiles) / (double(sm_count()) * per_sm);
   if (waves < 1.0) cost *= 1.0 + 0.15 * (1.0 - waves) * double(d.c) * d.n / (16.0 * d.nthr);
   return cost;
 }
