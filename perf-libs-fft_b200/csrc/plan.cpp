@@ -862,13 +862,6 @@ std::unique_ptr<Node> make_c2c_node(int64_t n, const Layout& lay, int dir, float
     auto p2 = make_pow2(n, lay, dir, scale, why);
     if (p2) return p2;
   }
-  // one to four members of a length with radix 11 or 13: the tile kernel ends
-  // sooner (us, tile / engine, back to back n=847 x 1 5.2 / 6.0, after another
-  // kernel 6.6 / 8.3, n=169 x 4 5.7 / 7.6, n=1040 x 1 7.0 / 7.6, x 8 equal)
-  if (unit && lay.howmany <= 4 && n <= 1040 && is_smooth(n) && (n % 11 == 0 || n % 13 == 0)) {
-    Addr ia{lay.idist, 0, 1, 1}, oa{lay.odist, 0, 1, 1};
-    if (auto t = make_tile(n, lay.howmany, ia, oa, dir, scale, false, why)) return t;
-  }
   // dense powers of two beyond the on-chip kernel keep the bulk-copy four-step
   if (!(unit && is_pow2(n) && n > 8192))
     if (auto t = make_mix_c2c<float2>(n, lay, dir, scale, false, why)) return t;
@@ -885,23 +878,22 @@ std::unique_ptr<Node> make_c2c_node(int64_t n, const Layout& lay, int dir, float
   return make_conv_node(n, lay, dir, scale, why);
 }
 
-// A few small transforms between other kernels: the tile kernel, whose code
-// is shorter, than the mixed-radix engine, which pays when its code is in the
-// SM's instruction cache (that is, back to back).  R2C of odd n in a graph, us,
-// tile / engine: n=33 x 1 6.6 / 8.9, n=225 x 1 8.4 / 12.7, n=39 x 8 7.0 / 10.0,
-// n=891 x 1 11.0 / 11.1, n=27 x 64 11.8 / 9.5; of 11 and 13 up to more
-// elements: n=65 x 64 10.5 / 12.7, n=363 x 8 11.6 / 12.1, n=847 x 8 equal.
-// Convolutions likewise: over the power of two (DCT-I of 363 x 1..64, inner
-// length 724, 7.5..8.4, and 9.0..10.2 over 1536 points).
+// A few members of a length whose stages are long ones, two radices of 11 and
+// more, between other kernels: the tile kernel, whose code is shorter, as the
+// SM's instruction cache is cold for it.  R2C and DCT-I of odd n, us, tile /
+// engine: inner length 143 = 13 x 11 x 4 11.4 / 14.4, 225 = 15 x 15 x 1 11.0 /
+// 14.4, 240 = 16 x 15 x 1 10.4 / 15.1, 429 = 13 x 11 x 3 x 4 13.8 / 16.5, 847 =
+// 11 x 11 x 7 x 2 13.7 / 14.4, x 4 16.4 / 14.4; of shorter stages 45 = 9 x 5 x 1
+// 10.3 / 8.4, 81 = 9 x 9 x 1 11.0 / 9.2, 700 = 10 x 10 x 7 x 1 13.7 / 10.3.
 std::unique_ptr<Node> make_c2c_inner_node(int64_t n, const Layout& lay, int dir, float scale, std::string* why) {
-  const int64_t top = n % 11 == 0 || n % 13 == 0 ? 4224 : 960;
   const bool pow2 = is_pow2(n) && n >= 64;
-  if (n > 8 && !pow2 && is_smooth(n) && n * lay.howmany <= top && lay.istride == 1 && lay.ostride == 1) {
-    Addr ia{lay.idist, 0, 1, 1}, oa{lay.odist, 0, 1, 1};
-    if (auto t = make_tile(n, lay.howmany, ia, oa, dir, scale, false, why)) return t;
+  if (!pow2 && n * lay.howmany <= 1716 && lay.istride == 1 && lay.ostride == 1) {
+    const std::vector<int> r = mix_radices(n, 16);
+    if (r.size() >= 2 && r[1] >= 11) {
+      Addr ia{lay.idist, 0, 1, 1}, oa{lay.odist, 0, 1, 1};
+      if (auto t = make_tile(n, lay.howmany, ia, oa, dir, scale, false, why)) return t;
+    }
   }
-  if (!is_smooth(n) && conv_fused_length(n) && lay.howmany <= 64)
-    if (auto c = make_conv_fused(n, lay, dir, scale, why, -1, 0, 0)) return c;
   return make_c2c_node(n, lay, dir, scale, 0, why);
 }
 

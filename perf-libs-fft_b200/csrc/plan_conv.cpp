@@ -344,7 +344,7 @@ static std::unique_ptr<Node> make_conv_list(int64_t n, const Layout& lay, int di
 }
 
 // e = 0: the default shape for the length (PLFFT_B200_CONV_E / _MINB / _G
-// override it), -1: that of the power of two, else the given shape
+// override it), else the given shape
 std::unique_ptr<Node> make_conv_fused(int64_t n, const Layout& lay, int dir, float scale, std::string* why, int e_req,
                                       int minb_req, int g_req) {
   if (std::getenv("PLFFT_B200_CONV_UNFUSED")) return nullptr;
@@ -352,7 +352,6 @@ std::unique_ptr<Node> make_conv_fused(int64_t n, const Layout& lay, int dir, flo
   if (m == 0) return nullptr;
   if (!e_req && !std::getenv("PLFFT_B200_CONV_E") && !std::getenv("PLFFT_B200_CONV_POW2"))
     if (auto l = make_conv_list(n, lay, dir, scale, why)) return l;
-  if (e_req < 0) e_req = 0;
   const bool rader = use_rader(n);
   const auto shapes = conv_fused_shapes(int(m));
   if (shapes.empty()) return nullptr;

@@ -111,10 +111,10 @@ struct F64RealNode : Node {
 std::unique_ptr<Node> make_fp64_c2c(int64_t n, const Layout& lay, int dir, double scale, std::string* why) {
   // 7-smooth n, and the 13-smooth ones the direct sums would take, but for the
   // shortest of these in batches that leave the chip idle: a short sum ends
-  // before the long radix does (us, sums / engine: n=13 x 64 2.4 / 4.0, x 2000
-  // 3.7 / 4.0, n=26 x 1000 3.3 / 4.2, x 2000 5.1 / 4.3, n=39 x 64 3.3 / 3.9,
-  // x 250 3.6 / 3.8, x 1000 4.4 / 3.9, n=44 x 64 3.6 / 3.3)
-  const bool sums = !smooth7(n) && ((n <= 26 && lay.howmany <= 1000) || (n <= 39 && lay.howmany <= 256));
+  // before the long radix does (us, sums / engine: n=13 x 16 3.5 / 3.1, x 32
+  // 3.5 / 4.1, x 1000 3.6 / 4.3, x 2000 3.7 / 4.0; n=26 x 64 4.1 / 4.3, x 1000
+  // 4.2 / 4.5, x 2000 5.1 / 4.3; n=33 x 64 4.2 / 3.8)
+  const bool sums = !smooth7(n) && n <= 26 && lay.howmany >= 32 && lay.howmany <= 1000;
   if (smooth7(n) || (is_smooth(n) && n <= kF64MaxOnChip && !sums))
     if (auto t = make_mix_c2c<double2>(n, lay, dir, scale, false, why)) return t;
   auto node = std::make_unique<F64C2CNode>();
