@@ -65,7 +65,9 @@ __global__ void __launch_bounds__(256) rd_pre(const ConvLaunch L, int64_t m0, in
   for (int64_t f = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; f < total; f += int64_t(gridDim.x) * blockDim.x) {
     const int64_t bl = flat_div(f, m, small);
     const int64_t q = f - bl * m;
-    L.work[f] = L.in[(m0 + bl) * L.idist + int64_t(L.perm_in[q]) * L.istride];
+    const float2* x = L.in + (m0 + bl) * L.idist;
+    L.work[f] = x[int64_t(L.perm_in[q]) * L.istride];
+    if (q == 0) L.x0[bl] = x[0];
   }
 }
 
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(256) rd_post(const ConvLaunch L, int64_t m0, i
     const int64_t bl = flat_div(f, m, small);
     const int64_t q = f - bl * m;
     const int64_t b = m0 + bl;
-    const float2 x0 = L.in[b * L.idist];
+    const float2 x0 = L.x0[bl];  // not the input: in place, element 0 is written here
     float2* y = L.out + b * L.odist;
     y[int64_t(L.perm_out[q]) * L.ostride] = cscale(cadd(x0, L.work[f]), s);
     if (q == 0) y[0] = cscale(cadd(x0, L.sum0[bl]), s);

@@ -144,6 +144,7 @@ struct ConvLaunch {
   float2* out;
   float2* work;   // [chunk][m]
   float2* sum0;   // [chunk] (Rader: A[0] per member)
+  float2* x0;     // [chunk] (Rader: input 0 per member)
   const float2* chirp;  // Bluestein w_k, k < n
   const float2* spec;   // convolution spectrum, m entries
   const int* perm_in;   // Rader g^q mod P

@@ -118,12 +118,11 @@ struct ConvNode : Node {
   }
 
   size_t work_bytes() const { return (size_t(chunk) * size_t(m) * sizeof(float2) + 255) & ~size_t(255); }
-  size_t sum_bytes() const { return (size_t(chunk) * sizeof(float2) + 255) & ~size_t(255); }
+  size_t sum_bytes() const { return (2 * size_t(chunk) * sizeof(float2) + 255) & ~size_t(255); }
   size_t workspace() const override {
     return work_bytes() + sum_bytes() + std::max(fwd->workspace(), bwd->workspace());
   }
-  // (Rader's last launch reads element 0 of each member again)
-  bool reads_batch_first() const override { return !rader && chunk >= lay.howmany; }
+  bool reads_batch_first() const override { return chunk >= lay.howmany; }
   int launches() const override {
     const int64_t chunks = (lay.howmany + chunk - 1) / chunk;
     return int(chunks * (3 + fwd->launches() + bwd->launches()));
@@ -138,6 +137,7 @@ struct ConvNode : Node {
     L.out = static_cast<float2*>(out);
     L.work = work;
     L.sum0 = sum0;
+    L.x0 = sum0 + chunk;
     L.chirp = chirp.as<float2>();
     L.spec = spec.as<float2>();
     L.perm_in = pin.as<int>();

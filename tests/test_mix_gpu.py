@@ -378,3 +378,16 @@ def test_four_step_members(n, hm, direction):
         untouched = torch.ones(y.numel(), dtype=torch.bool, device="cuda")
         torch.as_strided(untouched, (hm, n), (o[1], o[0])).fill_(False)
         assert bool((y[untouched] == 7.0).all()), "wrote outside the members"
+
+
+# long Rader and Bluestein transforms in place: element 0 of a member is an
+# output that other CTAs once read as the input
+@pytest.mark.parametrize("n,hm", [(12289, 1), (12289, 9), (40961, 3), (9001, 9)])
+def test_long_convolution_in_place(n, hm):
+    for s, d in [(1, n), (hm, 1)]:
+        x = seeded_complex(n * hm, n)
+        plan = plfft.make_plan("c2c", n, hm, s, d, s, d, alias=plfft.IoAlias.MAY_ALIAS)
+        buf = to_dev(x)
+        plan.execute(buf.data_ptr(), buf.data_ptr())
+        ref = np.fft.fft(gather(x, hm, d, n, s).astype(np.complex128))
+        assert oracle.rel_l2(gather(buf.cpu().numpy(), hm, d, n, s), ref) <= oracle.fp32_tol(n), plan.describe()
